@@ -735,7 +735,7 @@ def run_ours(args):
                 "d2h_bytes_per_step": W * H * 4, "latency_ms": {"p50": pct(lat_e, 50), "p99": pct(lat_e, 99)}},
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved / peak, 5), "traffic": ROOFLINE_TRAFFIC.get(args.config),
-                     "kernel": "render_pixels_kernel" if gc.render_tuning()[0] == 1 else "render_kernel",
+                     "kernel": "render_kernel",
                      "peak_kind": peak_kind, "algorithmic_bytes_per_launch": int(algo),
                      "launch_ms": round(render_ms, 4), "launch_ms_without_empty_skip": round(render_ms_noskip, 4),
                      "touched_bricks": int(touched), "samples_per_launch": int(samples),

@@ -43,6 +43,7 @@ struct LevelTables {
     uint32_t bb[kMaxCacheLevels][3];      // big-brick size (in bricks) of the level's volume
     float nbf[kMaxCacheLevels][3];        // nb and vvox as floats (exact: both < 2^24), for the
     float vvoxf[kMaxCacheLevels][3];      // ray caster's per-sample page walk
+    float cell[kMaxCacheLevels][3];       // a brick's edge in the ray caster's normalized coordinates
     uint32_t pt_off[kMaxCacheLevels];     // two-level directory: x offset of each level's words
 };
 
@@ -135,6 +136,7 @@ struct ViewParams {
     uint32_t nlevels;                   // levels of the view's volume
     uint32_t eb;                        // bytes per voxel of the view's volume
     uint32_t fallback;                  // sample a coarser mapped level where a brick is missing (preview)
+    float cell_margin, run_margin;      // margins of the ray caster's run through one brick (run_bound)
     uint32_t skip_empty;                // step through invisible bricks without sampling (DVR, one channel)
     unsigned long long visible;         // bins the view's transfer function can make visible
     uint32_t mark_done;                 // batched passes: a finished ray leaves -1 - t in tbuf and
@@ -258,7 +260,7 @@ void launch_unmark_in_flight(const uint4 *list, uint32_t n, const LevelTables &l
 void launch_completude(const float4 *slot_vpos, uint32_t nslots, uint32_t *count, cudaStream_t s);
 
 // Ray caster (render.cu).  Launch configuration of the ray caster, process
-// wide: scheduler 0 = one 8x4 tile per warp, 1 = per-lane pixel refill;
+// wide: scheduler (0 and 1 launch the same kernel, one ray tile per warp);
 // threads per block; blocks per SM cap (0 = occupancy limit).
 struct RenderTuning {
     uint32_t scheduler = 1;
@@ -270,15 +272,15 @@ struct RenderTuning {
 };
 RenderTuning &render_tuning();
 // Ray-caster kernels of a voxel kind (1, 2, 4 bytes; 0 mixed widths; 0x202
-// two 8-bit channels), scheduler and brick size (16 and 32 have kernels
+// two 8-bit channels) and brick size (16 and 32 have kernels
 // compiled for them; a two-level page directory has kernels of its own),
 // from the exact build (render.cu) or the fast build (render_fast.cu);
 // nullptr for an unsupported kind.
 namespace exact {
-void *march_kernel(uint32_t kind, bool pixels, uint32_t brick_size, bool two_level);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level);
 }
 namespace fast {
-void *march_kernel(uint32_t kind, bool pixels, uint32_t brick_size, bool two_level);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level);
 }
 // Fills ViewParams::visible of n device views from their transfer functions.
 void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s);

@@ -220,6 +220,7 @@ static void build_tables(gc_cache *C) {
                 lt.vvoxf[l][a] = static_cast<float>(lt.vvox[l][a]);
                 lt.ior[l][a] = static_cast<float>(L.initial[k][a]) / static_cast<float>(L.real[k][a]);
                 lt.bb[l][a] = V.desc.big_brick_size[a];
+                lt.cell[l][a] = 1.0f / (lt.ior[l][a] * lt.nbf[l][a]);
             }
             lt.eb[l] = V.desc.encoded_bytes;
             off += L.nb_bricks[k][0];
@@ -744,6 +745,14 @@ static void fill_view(const gc_cache *C, const gc_view &in, ViewParams &out) {
     const float bsy = in.bbox_max[1] - in.bbox_min[1];
     const float bsz = in.bbox_max[2] - in.bbox_min[2];
     const float bmin = std::min(bsx, std::min(bsy, bsz));
+    // twice the roundings of a ray's run through one brick, at most 7 (B - 2c) /
+    // bmin steps of half a voxel: half an ulp of the box's largest coordinate
+    // (at least 1) and of t a step (run_bound)
+    float extent = 1.0f;
+    for (int a = 0; a < 3; ++a) extent = std::max(extent, std::max(std::fabs(in.bbox_min[a]), std::fabs(in.bbox_max[a])));
+    const float run_steps = 7.0f * static_cast<float>(C->Beff) / bmin + 4.0f, half_ulp = 5.9604645e-8f;
+    out.cell_margin = 2.0f * (8.0f + run_steps * extent) * half_ulp;
+    out.run_margin = 2.0f * (4.0f + run_steps) * half_ulp;
     const gc_layout &L = V.layout;
     out.level_base = V.level_base;
     out.nlevels = L.nb_levels;

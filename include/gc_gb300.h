@@ -518,11 +518,11 @@ int gc_render(gc_cache_t cache, const gc_view *view, void *stream);
 int gc_render_batch(gc_cache_t cache, const gc_view *views, uint32_t n, void *stream);
 
 /* Launch configuration of the ray caster (process-wide; results do not
- * depend on it): scheduler 0 = a warp marches one ray tile at a time,
- * 1 = each lane refills from the pixel queue when its ray ends; tile width
- * 4, 8, 16 or 32 (a warp tile is tile_w x 32/tile_w pixels); threads per
- * block 64, 128 or 256; blocks per SM cap (0 = occupancy limit).  Chosen by
- * the autotuner of the Python host (gcgb300.autotune_render). */
+ * depend on it): scheduler 0 or 1 (the same kernel: each warp marches one
+ * ray tile at a time); tile width 4, 8, 16 or 32 (a warp tile is tile_w x
+ * 32/tile_w pixels); threads per block 64, 128 or 256; blocks per SM cap (0 =
+ * occupancy limit).  Chosen by the autotuner of the Python host
+ * (gcgb300.autotune_render). */
 int gc_render_tuning_set(uint32_t scheduler, uint32_t tile_w, uint32_t threads, uint32_t blocks_per_sm);
 int gc_render_tuning_get(uint32_t out[4]);
 /* Arithmetic of the ray caster (process-wide).  GC_RENDER_EXACT (default):

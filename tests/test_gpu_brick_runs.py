@@ -1,0 +1,84 @@
+"""The ray caster's runs through one brick (no page walk between the samples of a
+brick the ray surely stays in): frame by frame against the FP32 oracle, which
+walks the page directory at every sample, bit for bit -- RGBA, t, colour state,
+usage, requests and the rest of the cache state.
+
+The cases are those where a run could leave its brick: boxes other than
+[-1, 1]^3, view matrices that scale the ray directions, rays along the axes,
+cameras inside the volume, bricks of every size, base steps shorter and longer
+than the level's steps (empty bricks), and thin volumes."""
+import numpy as np
+import pytest
+
+import scenario
+from test_gpu_render import Scene
+
+pytestmark = pytest.mark.gpu
+
+
+def axis_camera(gc, axis, distance):
+    eye = [0.0, 0.0, 0.0]
+    eye[axis] = distance
+    return gc.look_at(eye, up=(0.0, 0.0, 1.0) if axis == 1 else (0.0, 1.0, 0.0))
+
+
+def scaled(m, s):
+    return [x if k % 4 == 3 else x * s for k, x in enumerate(m)]
+
+
+CASES = {
+    # name: (size, bpc, B, c, camera, empty threshold, view arguments)
+    "large_box": ((64, 64, 64), 1, 16, 1, lambda gc: scenario.orbit_camera(gc, 1, 12, 5.0), None,
+                  dict(bbox_min=(-3.0, -1.5, -2.0), bbox_max=(2.5, 3.0, 3.0))),
+    "small_box": ((64, 48, 64), 2, 16, 1, lambda gc: scenario.orbit_camera(gc, 2, 12, 1.2), None,
+                  dict(bbox_min=(-0.3, -0.4, -0.25), bbox_max=(0.35, 0.3, 0.4), sampler=1)),
+    "short_directions": ((64, 64, 64), 1, 16, 1, lambda gc: scaled(scenario.orbit_camera(gc, 1, 12, 2.4), 0.03), None,
+                         dict()),
+    "long_directions": ((64, 64, 64), 1, 16, 1, lambda gc: scaled(scenario.orbit_camera(gc, 1, 12, 2.4), 2.5), None,
+                        dict()),
+    "along_x": ((64, 64, 64), 1, 8, 1, lambda gc: axis_camera(gc, 0, 2.2), None, dict(focal=1e6)),
+    "along_y": ((64, 64, 64), 2, 8, 2, lambda gc: axis_camera(gc, 1, -2.2), None, dict(focal=1e6, mode=1)),
+    "along_z": ((64, 64, 64), 1, 16, 1, lambda gc: axis_camera(gc, 2, 30.0), None, dict(focal=30.0)),
+    "inside": ((96, 64, 64), 2, 16, 1, lambda gc: gc.look_at((0.1, -0.2, 0.3), (0.9, 0.4, -0.6)), None,
+               dict(focal=0.8)),
+    "brick_4": ((32, 32, 32), 1, 4, 1, lambda gc: scenario.orbit_camera(gc, 4, 12, 2.6), None, dict()),
+    "brick_64": ((96, 128, 96), 1, 64, 3, lambda gc: scenario.orbit_camera(gc, 5, 12, 2.6), None, dict()),
+    "thin": ((128, 24, 40), 1, 16, 1, lambda gc: scenario.orbit_camera(gc, 2, 12, 2.2), None, dict()),
+    "empty_short_base": ((64, 64, 64), 1, 16, 1, lambda gc: scenario.orbit_camera(gc, 3, 12, 2.4), 24.0,
+                         dict(tstep=0.003)),
+    "empty_long_base": ((64, 64, 64), 1, 16, 1, lambda gc: scenario.orbit_camera(gc, 3, 12, 2.4), 24.0,
+                        dict(tstep=0.11)),
+}
+
+
+@pytest.mark.parametrize("case", sorted(CASES))
+def test_runs_match_the_walked_march(gc, orc, torch_cuda, case):
+    size, bpc, B, c, cam, empty, kw = CASES[case]
+    s = Scene(gc, orc, torch_cuda, size, bpc, B, c, (1, 1, 1), (8, 8, 8) if B < 64 else (3, 3, 3), 27)
+    if empty is not None:
+        d = scenario.gpu_volume(gc, torch_cuda, size, bpc, 21, 6)
+        _, _, keys = gc.pre_process(s.vol, s.layout, d, empty_threshold=empty)
+        assert keys
+        s.cm.set_source_host(s.store, s.offs, keys)
+        s.oc.set_source(s.ref, s.offs, keys)
+    tf = scenario.bumps_tf(3)
+    tf_dev = torch_cuda.from_numpy(tf.reshape(-1)).cuda()
+    W, H = 45, 38
+    g, o = s.buffers(W, H)
+    v = s.view(cam(gc), W, H, tf_dev, 256, g, **dict(dict(early_alpha=0.99), **kw))
+    converged, marched = False, 0
+    for frame in range(60):
+        s.cm.render(v)
+        s.oc.render(v, tf, *o)
+        torch_cuda.cuda.synchronize()
+        tag = f"{case}, frame {frame}"
+        assert np.array_equal(g[0].cpu().numpy().view(np.uint32), o[0].view(np.uint32)), tag
+        assert np.array_equal(g[1].cpu().numpy(), o[1]), tag
+        assert np.array_equal(g[2].cpu().numpy(), o[2]), tag
+        converged = s.cm.update()
+        assert converged == s.oc.update(), tag
+        s.compare_cache(tag)
+        if converged:
+            break
+    marched = s.cm.stats().rays_marched
+    assert marched > 0 and s.cm.stats().bricks_installed > 0
