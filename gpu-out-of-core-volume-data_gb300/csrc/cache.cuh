@@ -136,6 +136,8 @@ struct ViewParams {
     uint32_t nlevels;                   // levels of the view's volume
     uint32_t eb;                        // bytes per voxel of the view's volume
     uint32_t fallback;                  // sample a coarser mapped level where a brick is missing (preview)
+    uint32_t skip_max;                  // maximum intensity, one channel: step through bricks that cannot
+                                        // raise the maximum
     float cell_margin, run_margin;      // margins of the ray caster's run through one brick (run_bound)
     uint32_t skip_empty;                // step through invisible bricks without sampling (DVR, one channel)
     unsigned long long visible;         // bins the view's transfer function can make visible

@@ -734,6 +734,10 @@ static void fill_view(const gc_cache *C, const gc_view &in, ViewParams &out) {
     out.tfh = in.tf_height > 0 ? in.tf_height : 1;
     // empty-space skipping: DVR of one channel through a 1D transfer function
     out.skip_empty = in.mode == GC_MODE_DVR && V.desc.channels == 1 ? render_tuning().skip_empty : 0u;
+    // and maximum intensity of one channel of integer voxels
+    out.skip_max = in.mode == GC_MODE_MOP && V.desc.channels == 1 && V.desc.encoded_bytes <= 2
+                       ? render_tuning().skip_empty
+                       : 0u;
     out.visible = ~0ull;  // filled from the transfer function on the device (view_bins_kernel)
     out.tf = in.tf;
     out.rgba = in.rgba;

@@ -543,7 +543,9 @@ int gc_render_precision_get(int *precision);
  * DVR view of a one-channel volume the value range its transfer function can
  * make visible; a ray steps through a brick with no visible value without
  * sampling it (the same t steps; samples there stay below the 0.001
- * compositing threshold).  No counterpart in the reference. */
+ * compositing threshold).  A maximum-intensity ray of a one-channel volume of
+ * integer voxels steps likewise through a brick whose range cannot raise its
+ * maximum.  No counterpart in the reference. */
 int gc_render_empty_skip(int enable);
 
 /* ------------------------------------------------------------------------ */

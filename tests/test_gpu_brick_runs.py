@@ -82,3 +82,53 @@ def test_runs_match_the_walked_march(gc, orc, torch_cuda, case):
             break
     marched = s.cm.stats().rays_marched
     assert marched > 0 and s.cm.stats().bricks_installed > 0
+
+
+@pytest.mark.parametrize("bpc,sampler", [(1, 0), (1, 1), (2, 0), (2, 1), (4, 1)])
+def test_maximum_intensity_skips_change_nothing(gc, torch_cuda, bpc, sampler):
+    """Bricks that cannot raise a ray's maximum are stepped through: image, t and
+    maximum equal those without skipping, bit for bit, with values at both ends
+    of the range (float voxels, which may lie outside [0, 1], are not skipped)."""
+    t = torch_cuda
+    n = 48
+    gen = t.Generator().manual_seed(7)
+    v = t.rand((n, n, n), generator=gen)
+    v = t.where(v < 0.3, t.zeros(()), t.where(v > 0.98, t.ones(()), v * 0.9))  # bins 0 .. 63
+    v[8:40, 8:40, 8:40] *= t.linspace(0.2, 1.0, 32)[:, None, None]
+    if bpc == 4:
+        d = (v * 3.0 - 1.0).reshape(-1).cuda()
+    else:
+        d = (v * (255 if bpc == 1 else 65535)).to(t.int32).to(t.uint8 if bpc == 1 else t.int16).reshape(-1).cuda()
+    vol = gc.volume_desc((n, n, n), 8, 1, bpc)
+    layout = gc.compute_layout(vol)
+    store, offs, _ = gc.pre_process(vol, layout, d)
+    tf = t.from_numpy(scenario.bumps_tf(3).reshape(-1)).cuda()
+    images, samples = [], []
+    for skip in (False, True):
+        cm = gc.CacheManager(vol, layout, (10, 10, 10), max_requests=1000)
+        cm.set_source_host(store, offs)
+        W, H = 53, 41
+        b = (t.zeros(W * H, dtype=t.int32, device="cuda"), t.zeros(W * H, device="cuda"),
+             t.zeros(W * H * 4, device="cuda"))
+        view = gc.make_view(scenario.orbit_camera(gc, 1, 12, 2.4), W, H, tf.data_ptr(), 256, b[0].data_ptr(),
+                            b[1].data_ptr(), b[2].data_ptr(), mode=gc.MODE_MOP, sampler=sampler)
+        gc.render_empty_skip(skip)
+        try:
+            for _ in range(60):
+                cm.render(view)
+                if cm.update():
+                    break
+            for x in b[1:]:
+                x.zero_()
+            before = cm.stats().samples
+            cm.render(view)
+            t.cuda.synchronize()
+            samples.append(cm.stats().samples - before)
+        finally:
+            gc.render_empty_skip(True)
+        images.append([x.cpu().numpy() for x in b])
+        cm.close()
+    for x, y in zip(*images):
+        assert np.array_equal(x, y)
+    assert images[0][2].any()
+    assert samples[1] == samples[0] if bpc == 4 else samples[1] < samples[0]
