@@ -279,16 +279,16 @@ RenderTuning &render_tuning();
 // from the exact build (render.cu) or the fast build (render_fast.cu);
 // nullptr for an unsupported kind.
 namespace exact {
-void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, bool few_rays);
 }
 namespace fast {
-void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, bool few_rays);
 }
 // Fills ViewParams::visible of n device views from their transfer functions.
 void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s);
 void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev,
-                   const ViewParams *views_host, uint32_t nviews, uint32_t total_tiles, uint32_t *queue,
-                   uint32_t *err, cudaStream_t s);
+                   const ViewParams *views_host, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
+                   uint32_t *queue, cudaStream_t s);
 
 // An executable CUDA graph of the batched launch (view-table copy + ray caster).
 struct RenderGraph {
@@ -305,7 +305,7 @@ struct RenderGraph {
     void reset();
 };
 void launch_render_graph(RenderGraph &g, const CacheView &cv, const LevelTables &lt, ViewParams *views_dev,
-                         const ViewParams *views_pinned, uint32_t nviews, uint32_t total_tiles, uint32_t *queue,
-                         cudaStream_t s);
+                         const ViewParams *views_pinned, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
+                         uint32_t *queue, cudaStream_t s);
 
 }  // namespace gc

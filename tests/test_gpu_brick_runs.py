@@ -132,3 +132,51 @@ def test_maximum_intensity_skips_change_nothing(gc, torch_cuda, bpc, sampler):
         assert np.array_equal(x, y)
     assert images[0][2].any()
     assert samples[1] == samples[0] if bpc == 4 else samples[1] < samples[0]
+
+
+@pytest.mark.parametrize("kind", ["u8", "u16", "f32", "two", "u8_two_level", "u8_b8"])
+@pytest.mark.parametrize("mode,sampler", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_launches_of_few_and_many_rays_agree(gc, torch_cuda, kind, mode, sampler):
+    """A launch of few rays takes more samples of a ray at a time than a launch of
+    many: the same views in launches of one view and of one batch (over 24 x 32
+    rays per SM) give the same image, t and colour state, bit for bit."""
+    t = torch_cuda
+    n, bpc, ch = 48, {"u16": 2, "f32": 4, "two": 2}.get(kind, 1), 2 if kind == "two" else 1
+    B = 8 if kind == "u8_b8" else 16
+    vol = gc.volume_desc((n, n, n), B, 1, bpc, ch)
+    layout = gc.compute_layout(vol)
+    if kind == "f32":
+        d = scenario.gpu_volume(gc, t, (n, n, n), 1, 5, 6).float().div_(255.0)
+    else:
+        d = scenario.gpu_volume(gc, t, (n, n, n), bpc // ch, 5, 6, channels=ch)
+    store, offs, _ = gc.pre_process(vol, layout, d)
+    cm = gc.CacheManager(vol, layout, (9, 9, 9), max_requests=700, pt_block=4 if kind == "u8_two_level" else 0,
+                         pt_slots=64 if kind == "u8_two_level" else 0)
+    cm.set_source_host(store, offs)
+    tf = scenario.tf2d(5) if ch == 2 else scenario.bumps_tf(3)
+    tf_dev = t.from_numpy(tf.reshape(-1)).cuda()
+    W, H, k = 181, 142, 8  # 8 views of 23 x 36 tiles
+    bufs = [(t.zeros(W * H, dtype=t.int32, device="cuda"), t.zeros(W * H, device="cuda"),
+             t.zeros(W * H * 4, device="cuda")) for _ in range(k)]
+    views = [gc.make_view(scenario.orbit_camera(gc, i, 2 * k, 1.3 + 0.1 * i), W, H, tf_dev.data_ptr(), tf.shape[-2],
+                          b[0].data_ptr(), b[1].data_ptr(), b[2].data_ptr(), focal=0.9, early_alpha=0.99, mode=mode,
+                          sampler=sampler, tf_height=tf.shape[0] if ch == 2 else 0) for i, b in enumerate(bufs)]
+    assert k * 23 * 36 > 24 * t.cuda.get_device_properties(0).multi_processor_count > 23 * 36
+    for _ in range(100):
+        cm.render_batch(views)
+        if cm.update():
+            break
+
+    def images(render):
+        for b in bufs:
+            for x in b:
+                x.zero_()
+        render()
+        t.cuda.synchronize()
+        return [x.cpu().numpy() for b in bufs for x in b]
+
+    one = images(lambda: [cm.render(v) for v in views])
+    many = images(lambda: cm.render_batch(views))
+    assert any(x.any() for x in one)
+    for x, y in zip(one, many):
+        assert np.array_equal(x, y)
