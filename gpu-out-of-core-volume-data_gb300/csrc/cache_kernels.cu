@@ -26,6 +26,7 @@
 
 #include "cache.cuh"
 #include "gc_internal.h"
+#include "value_range.cuh"
 
 namespace gc {
 
@@ -320,8 +321,19 @@ __global__ void install_evict_kernel(InstallArgs a, const LevelTables lt) {
 // over its voxels (covering included), normalized like the samplers, widened
 // by one bin on either side.  `at(v)` gives the address of voxel v; one
 // block per brick (up to 256 threads); the result is valid in thread 0.
-// The block's value bins from each thread's min and max (normalized like the
-// samplers); the result is valid in thread 0.
+// The value bins of the range [lo, hi] (normalized like the samplers), widened
+// by one bin on either side.
+__device__ __forceinline__ unsigned long long bins_of_range(float lo, float hi) {
+    auto bin = [](float x) {
+        const float f = floorf(x * static_cast<float>(kValueBins));
+        return f < 0.f ? 0 : (f > kValueBins - 1.f ? static_cast<int>(kValueBins) - 1 : static_cast<int>(f));
+    };
+    const int b0 = max(bin(lo) - 1, 0), b1 = min(bin(hi) + 1, static_cast<int>(kValueBins) - 1);
+    const unsigned long long upto = b1 >= 63 ? ~0ull : ((1ull << (b1 + 1)) - 1ull);
+    return upto & ~((1ull << b0) - 1ull);
+}
+// The block's value bins from each thread's min and max; the result is valid in
+// thread 0.
 __device__ unsigned long long block_bins_from(float lo, float hi) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -335,21 +347,12 @@ __device__ unsigned long long block_bins_from(float lo, float hi) {
         s_hi[warp] = hi;
     }
     __syncthreads();
-    unsigned long long bins = 0;
-    if (threadIdx.x == 0) {
-        for (uint32_t w = 1; w < (blockDim.x + 31) / 32; ++w) {
-            lo = fminf(lo, s_lo[w]);
-            hi = fmaxf(hi, s_hi[w]);
-        }
-        auto bin = [](float x) {
-            const float f = floorf(x * static_cast<float>(kValueBins));
-            return f < 0.f ? 0 : (f > kValueBins - 1.f ? static_cast<int>(kValueBins) - 1 : static_cast<int>(f));
-        };
-        const int b0 = max(bin(lo) - 1, 0), b1 = min(bin(hi) + 1, static_cast<int>(kValueBins) - 1);
-        const unsigned long long upto = b1 >= 63 ? ~0ull : ((1ull << (b1 + 1)) - 1ull);
-        bins = upto & ~((1ull << b0) - 1ull);
+    if (threadIdx.x != 0) return 0;
+    for (uint32_t w = 1; w < (blockDim.x + 31) / 32; ++w) {
+        lo = fminf(lo, s_lo[w]);
+        hi = fmaxf(hi, s_hi[w]);
     }
-    return bins;
+    return bins_of_range(lo, hi);
 }
 template <class At>
 __device__ unsigned long long block_value_bins(uint32_t nvox, uint32_t eb, At at) {
@@ -416,13 +419,84 @@ __global__ void __launch_bounds__(256) brick_bins_kernel(const uint8_t *__restri
     if (threadIdx.x == 0) bins[i] = m;
 }
 
+// The same for bricks of whole 16-byte row chunks in a 16-byte aligned level: G
+// threads per brick read it 16 bytes a lane with four loads in flight.  Bound by
+// the read of the store.  A warp per brick (G = 32) up to 16 KiB, so that no
+// block barrier follows a brick's few loads; a block above, where one warp would
+// take 64 KiB bricks in 32 dependent turns.  The bricks of a 768^3 u16 volume
+// (16^3, 1.36 GB): 1970 -> 185 us, 7.4 TB/s.
+template <int EB, int G>
+__global__ void __launch_bounds__(256) brick_bins_vec_kernel(const uint8_t *__restrict__ level, uint32_t n,
+                                                             uint32_t nbx, uint32_t nby, uint32_t gbx, uint32_t gby,
+                                                             uint32_t bb0, uint32_t bb1, uint32_t bb2, uint32_t B,
+                                                             uint32_t cpr, unsigned long long *bins) {
+    const uint32_t i = G == 256 ? blockIdx.x : blockIdx.x * (256 / G) + threadIdx.x / G;
+    const uint32_t lane = threadIdx.x % G;
+    if (i >= n) return;  // the same for the G threads of the brick
+    const uint32_t x = i % nbx, r = i / nbx, y = r % nby, z = r / nby;
+    const uint32_t gx = x / bb0, gy = y / bb1, gz = z / bb2;
+    const uint32_t chunks = B * B * cpr;  // per brick
+    const uint64_t big = (static_cast<uint64_t>(gz) * gby + gy) * gbx + gx;
+    const bool whole = bb0 == 1 && bb1 == 1;  // the brick's chunks lie one after the other
+    const uint4 *p = reinterpret_cast<const uint4 *>(level) + big * (static_cast<uint64_t>(bb0) * bb1 * bb2 * chunks) +
+                     ((static_cast<uint64_t>(z - gz * bb2) * B * (bb1 * B) + (y - gy * bb1) * B) * bb0 + (x - gx * bb0)) * cpr;
+    ValueRange<EB> range;
+    for (uint32_t c0 = lane; c0 < chunks; c0 += 4u * G) {
+        uint4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t c = c0 + u * G;
+            if (c < chunks) {
+                uint64_t at = c;
+                if (!whole) {
+                    const uint32_t row = c / cpr, q = c - row * cpr, lz = row / B, ly = row - lz * B;
+                    at = static_cast<uint64_t>(lz * (bb1 * B) + ly) * (bb0 * cpr) + q;
+                }
+                v[u] = __ldcs(p + at);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (c0 + u * G < chunks) range.add(v[u]);
+    }
+    float lo = 3.4e38f, hi = -3.4e38f;
+    if (lane < chunks) range.normalized(lo, hi);
+    if constexpr (G == 256) {
+        const unsigned long long m = block_bins_from(lo, hi);
+        if (lane == 0) bins[i] = m;
+    } else {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane == 0) bins[i] = bins_of_range(lo, hi);
+    }
+}
+
 void launch_brick_bins(const uint8_t *level, const uint32_t nb[3], const uint32_t nbig[3], const uint32_t bb[3],
                        uint32_t B, uint32_t eb, unsigned long long *bins, cudaStream_t s) {
     const uint64_t n = static_cast<uint64_t>(nb[0]) * nb[1] * nb[2];
     if (n == 0) return;
     GC_REQUIRE(n < (1ull << 31), "too many bricks in one level");
-    brick_bins_kernel<<<static_cast<uint32_t>(n), 256, 0, s>>>(level, nb[0], nb[1], nb[2], nbig[0], nbig[1], bb[0],
-                                                              bb[1], bb[2], B, eb, bins);
+    const uint32_t n32 = static_cast<uint32_t>(n);
+    if ((B * eb) % 16 == 0 && B <= 512 && reinterpret_cast<uintptr_t>(level) % 16 == 0) {
+        const uint32_t cpr = B * eb / 16;
+        const bool warp = B * B * cpr <= 1024;  // 16 KiB
+        auto go = [&](auto kernel) {
+            kernel<<<warp ? div_up(n32, 8u) : n32, 256, 0, s>>>(level, n32, nb[0], nb[1], nbig[0], nbig[1], bb[0], bb[1],
+                                                               bb[2], B, cpr, bins);
+        };
+        if (eb == 1)
+            warp ? go(brick_bins_vec_kernel<1, 32>) : go(brick_bins_vec_kernel<1, 256>);
+        else if (eb == 2)
+            warp ? go(brick_bins_vec_kernel<2, 32>) : go(brick_bins_vec_kernel<2, 256>);
+        else
+            warp ? go(brick_bins_vec_kernel<4, 32>) : go(brick_bins_vec_kernel<4, 256>);
+    } else {
+        brick_bins_kernel<<<n32, 256, 0, s>>>(level, nb[0], nb[1], nb[2], nbig[0], nbig[1], bb[0], bb[1], bb[2], B, eb,
+                                             bins);
+    }
     GC_CUDA(cudaGetLastError());
     count_launch();
 }

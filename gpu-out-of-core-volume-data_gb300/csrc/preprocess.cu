@@ -8,6 +8,7 @@
 
 #include "cache.cuh"
 #include "gc_internal.h"
+#include "value_range.cuh"
 
 namespace gc {
 
@@ -508,6 +509,51 @@ __global__ void __launch_bounds__(256) empty_kernel(const uint8_t *__restrict__ 
     }
 }
 
+// The same for big bricks of whole 16-byte chunks, 16-byte aligned: G threads per
+// big brick, 16 bytes a lane with four loads in flight, ended by a vote once a
+// value reaches the threshold (an integer brick is empty when its largest value
+// is below it).  Bound by the read of the bricks that are empty; the first turn
+// (2 KiB with a warp, 16 KiB with a block) is read of every brick.  A warp per
+// big brick below 32 KiB (the reads of a turn fit the brick), a block above.
+// The bricks of a 768^3 u16 volume (16^3, 1.36 GB): 712 -> 66 us.
+template <int CB, int G>
+__global__ void __launch_bounds__(256) empty_vec_kernel(const uint4 *__restrict__ bricks, uint64_t nbig,
+                                                        uint64_t chunks, float threshold,
+                                                        uint8_t *__restrict__ flags) {
+    constexpr uint32_t kPer = 256 / G;
+    const uint32_t lane = threadIdx.x % G;
+    for (uint64_t b = static_cast<uint64_t>(blockIdx.x) * kPer + threadIdx.x / G; b < nbig;
+         b += static_cast<uint64_t>(gridDim.x) * kPer) {
+        const uint4 *p = bricks + b * chunks;
+        bool nonempty = false;
+        for (uint64_t c0 = 0; c0 < chunks && !nonempty; c0 += 4u * G) {
+            uint4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint64_t c = c0 + u * G + lane;
+                if (c < chunks) v[u] = __ldcs(p + c);
+            }
+            ValueRange<CB> range;
+            bool over = false, any = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c0 + u * G + lane < chunks) {
+                    any = true;
+                    if constexpr (CB == 4) {
+                        over = over || !(__uint_as_float(v[u].x) < threshold) || !(__uint_as_float(v[u].y) < threshold) ||
+                               !(__uint_as_float(v[u].z) < threshold) || !(__uint_as_float(v[u].w) < threshold);
+                    } else {
+                        range.add(v[u]);
+                    }
+                }
+            }
+            if constexpr (CB != 4) over = any && !(static_cast<float>(range.highest()) < threshold);
+            nonempty = G == 256 ? __syncthreads_or(over) != 0 : __any_sync(0xffffffffu, over) != 0;
+        }
+        if (lane == 0) flags[b] = nonempty ? 0 : 1;
+    }
+}
+
 }  // namespace gc
 
 using namespace gc;
@@ -600,6 +646,26 @@ int gc_bricks_empty(const void *bricks, uint64_t nb_big_bricks, const gc_volume_
         const uint64_t values = B * B * B * vol->big_brick_size[0] * vol->big_brick_size[1] *
                                 vol->big_brick_size[2] * vol->channels;
         if (nb_big_bricks == 0) return;
+        const uint32_t cb = channel_bytes(*vol);
+        const uint64_t bytes = values * cb;
+        if (bytes % 16 == 0 && reinterpret_cast<uintptr_t>(bricks) % 16 == 0 && (cb == 1 || cb == 2 || cb == 4)) {
+            const bool warp = bytes < (32u << 10);
+            const uint64_t blocks = std::min<uint64_t>(warp ? (nb_big_bricks + 7) / 8 : nb_big_bricks,
+                                                       static_cast<uint64_t>(sm_count()) * 64);
+            auto go = [&](auto kernel) {
+                kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
+                    static_cast<const uint4 *>(bricks), nb_big_bricks, bytes / 16, threshold, flags);
+            };
+            if (cb == 1)
+                warp ? go(empty_vec_kernel<1, 32>) : go(empty_vec_kernel<1, 256>);
+            else if (cb == 2)
+                warp ? go(empty_vec_kernel<2, 32>) : go(empty_vec_kernel<2, 256>);
+            else
+                warp ? go(empty_vec_kernel<4, 32>) : go(empty_vec_kernel<4, 256>);
+            GC_CUDA(cudaGetLastError());
+            count_launch();
+            return;
+        }
         const uint64_t grid = std::min<uint64_t>(nb_big_bricks, static_cast<uint64_t>(sm_count()) * 16);
         empty_kernel<<<static_cast<unsigned>(grid), 256, 0, as_stream(stream)>>>(
             static_cast<const uint8_t *>(bricks), nb_big_bricks, values, channel_bytes(*vol), threshold,
