@@ -4,6 +4,7 @@
 // per chunk (GcCore/src/cuda/libPreprocessor/Mipmapper.cu:401-578) and bricks
 // on the CPU with one seek+read per brick row
 // (GcCore/src/libPreprocessor/Bricker_v2.cpp:79-252).
+#include <algorithm>
 #include <cstring>
 
 #include "cache.cuh"
@@ -370,81 +371,316 @@ __device__ __forceinline__ uint4 window16(uint4 a, uint4 b, uint32_t s) {
                       __funnelshift_r(v3, v4, r));
 }
 
-// Row-mapped bricker (p.fast and at most 32 16-byte chunks per brick row): a
-// warp takes a run of nb = 32 / cpr bricks adjacent along x (one (sy, sz)
-// brick row), lane q holding chunk q % cpr of brick q / cpr, and walks the
-// B x B rows of the run.  Each row step reads one contiguous span of the
-// level row (nb bricks' windows, about 32 chunks, each fetched by at most two
-// lanes and merged in L1) and writes each brick's row chunk with one 16-byte
-// store.  Rows are whole 16-byte chunks of the level (row bytes a multiple of
-// 16, aligned level), so a chunk lies entirely inside or outside the row:
-// chunks outside read as zero, which is the bricker's value there (outside
-// the level); rows outside the level and unvisited bricks store zeros.  Row
-// steps go four at a time, their loads issued before their stores.
-__global__ void __launch_bounds__(256) brick_rows_kernel(const uint8_t *__restrict__ level,
-                                                         uint8_t *__restrict__ out, BrickParams p, uint32_t ngx) {
-    const uint32_t B = p.B, eb = p.eb;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t nb = 32u >> p.cpr_shift;
-    const uint32_t j = lane >> p.cpr_shift, k = lane & ((1u << p.cpr_shift) - 1u);
-    const uint32_t nsx = p.nbig[0] * p.BB[0], nsy = p.nbig[1] * p.BB[1], nsz = p.nbig[2] * p.BB[2];
+// Bytes [s, s + 8) of the 16-byte pair (a, b) for a per-lane s in 0..7.
+__device__ __forceinline__ uint2 window8(uint2 a, uint2 b, uint32_t s) {
+    const bool w1 = (s & 4u) != 0u;
+    const uint32_t v0 = w1 ? a.y : a.x, v1 = w1 ? b.x : a.y, v2 = w1 ? b.y : b.x;
+    const uint32_t r = (s & 3u) * 8u;
+    return make_uint2(__funnelshift_r(v0, v1, r), __funnelshift_r(v1, v2, r));
+}
+
+// x / d for x, d < 2^16: a shift, or a multiply-high by ceil(2^32 / d).
+struct SmallDiv {
+    uint32_t m = 0, shift = 0;
+    SmallDiv() = default;
+    explicit SmallDiv(uint32_t d) {
+        if ((d & (d - 1u)) == 0u)
+            while ((1u << shift) < d) ++shift;
+        else
+            m = static_cast<uint32_t>(((1ull << 32) + d - 1u) / d);
+    }
+    __device__ __forceinline__ uint32_t operator()(uint32_t x) const { return m ? __umulhi(x, m) : x >> shift; }
+};
+
+// One launch of the slab bricker.
+struct SlabParams {
+    BrickParams p;
+    uint32_t nb;             // bricks of a slab, adjacent along x
+    uint32_t ngx;            // slabs along x
+    uint32_t zparts, zlen;   // blocks that share a slab's slices, and slices of each
+    uint32_t cprow;          // 16-byte chunks copied of each source row
+    uint32_t pitch;          // bytes between the rows of a slice in shared memory
+    uint32_t stages;
+    uint32_t cpr;            // output chunks per brick row
+    uint64_t items;
+    SmallDiv by_cprow, by_brick, by_cpr;  // / cprow, / (B cpr), / cpr
+};
+
+// A 16-byte asynchronous copy of n <= 16 source bytes, the rest zeros.
+__device__ __forceinline__ void copy16_async(uint32_t dst, const uint8_t *src, uint32_t n) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Waits until at most `left` (0 to 3) of this thread's newest copy groups are in flight.
+__device__ __forceinline__ void copies_wait(uint32_t left) {
+    if (left == 0)
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else if (left == 1)
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else if (left == 2)
+        asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else
+        asm volatile("cp.async.wait_group 3;" ::: "memory");
+}
+
+// Slab bricker, for brick rows of whole CH-byte chunks (16, or 8 for 8-byte rows)
+// and levels of any row length.  A block takes a slab of nb bricks adjacent along
+// x and walks the slab's slices (one z of the level each): the B source rows of a
+// slice come into shared memory as aligned 16-byte asynchronous copies, several
+// slices ahead, and go out as whole brick rows -- consecutive lanes write
+// consecutive chunks of one brick, each cut out of its row at any byte offset
+// (rows of a level need not be multiples of 16 bytes apart: every row has its own
+// offset in its first chunk).  Copies are cut at the end of the row (zeros follow,
+// the bricker's value there), rows outside the level are zeros, bytes left of the
+// row are masked on the way out, unvisited bricks are zeros.
+//
+// Bound by HBM: the level is read once (slab edges again from L2) and the bricks,
+// (B / (B - 2c))^3 times its size, written once.  A slab is about 512 output
+// chunks a slice, so that a row's copies are several hundred bytes; small levels
+// share a slab's slices among blocks until the SMs are filled, because a block's
+// slices follow one another.  768^3 u16, 16^3 bricks, level 0 (2.27 GB): 450 us with
+// a warp per run of bricks straight from the level (32-byte pieces of 16 bricks a
+// store) -> 347 us, 6.5 TB/s; its level of 8 bricks 51 -> 4.4 us; level 0 of a
+// 381x347x291 u8 volume (rows of odd length) 310 us voxel by voxel -> 25 us.
+template <int CH>
+__global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restrict__ level, uint8_t *__restrict__ out,
+                                                         const SlabParams sp) {
+    extern __shared__ __align__(128) uint8_t slab_smem[];
+    const BrickParams &p = sp.p;
+    const uint32_t B = p.B, eb = p.eb, tid = threadIdx.x;
+    const uint32_t nsx = p.nbig[0] * p.BB[0], nsy = p.nbig[1] * p.BB[1];
     const uint32_t bvx = p.BB[0] * B, bvy = p.BB[1] * B;
     const uint64_t big_bytes = static_cast<uint64_t>(bvx) * bvy * (p.BB[2] * B) * eb;
-    const uint64_t row_bytes = static_cast<uint64_t>(p.D[0]) * eb;
-    const int64_t row_chunks = static_cast<int64_t>(row_bytes >> 4);
     const uint64_t drow = static_cast<uint64_t>(bvx) * eb;  // output row stride
-    const uint32_t nseg_xy = ngx * nsy;
-    const uint64_t nseg = static_cast<uint64_t>(nseg_xy) * nsz;
-    const uint32_t nrows = B * B;
-    const uint64_t gwarp = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (uint64_t seg = gwarp; seg < nseg; seg += nwarps) {
-        const uint32_t sz = static_cast<uint32_t>(seg / nseg_xy);
-        const uint32_t rem = static_cast<uint32_t>(seg - static_cast<uint64_t>(sz) * nseg_xy);
-        const uint32_t sy = rem / ngx, g = rem - sy * ngx;
-        const uint32_t sx = g * nb + j;
-        const bool valid = sx < nsx;
+    const int64_t row_bytes = static_cast<int64_t>(p.D[0]) * eb, plane = row_bytes * p.D[1];
+    const uint32_t slice_bytes = B * sp.pitch, ncopy = B * sp.cprow;
+    const uint32_t smem = static_cast<uint32_t>(__cvta_generic_to_shared(slab_smem));
+    for (uint64_t item = blockIdx.x; item < sp.items; item += gridDim.x) {
+        const uint32_t zp = static_cast<uint32_t>(item % sp.zparts);
+        const uint64_t slab = item / sp.zparts;
+        const uint32_t g = static_cast<uint32_t>(slab % sp.ngx);
+        const uint32_t rest = static_cast<uint32_t>(slab / sp.ngx), sy = rest % nsy, sz = rest / nsy;
+        const uint32_t sx0 = g * sp.nb, nbx = min(sp.nb, nsx - sx0);
         const bool yz_vis = static_cast<uint64_t>(sy) * p.Beff < p.D[1] && static_cast<uint64_t>(sz) * p.Beff < p.D[2];
-        const bool x_vis = static_cast<uint64_t>(sx) * p.Beff < p.D[0];
-        // this lane's source window in any row: bytes [o, o + 16), o = its
-        // chunk's first voxel byte (negative in the covering left of x = 0)
-        const int64_t o = (static_cast<int64_t>(sx) * p.Beff - p.c) * eb + 16 * static_cast<int64_t>(k);
-        const int64_t ca = o >> 4;  // floor
-        const uint32_t s = static_cast<uint32_t>(o - ca * 16);
-        const bool a_in = x_vis && ca >= 0 && ca < row_chunks;
-        const bool b_in = x_vis && s != 0u && ca + 1 >= 0 && ca + 1 < row_chunks;
-        const uint32_t gx = valid ? sx / p.BB[0] : 0u, gy = sy / p.BB[1], gz = sz / p.BB[2];
-        const uint32_t ix = sx - gx * p.BB[0], iy = sy - gy * p.BB[1], iz = sz - gz * p.BB[2];
-        const uint64_t big = (static_cast<uint64_t>(gz) * p.nbig[1] + gy) * p.nbig[0] + gx;
-        uint8_t *dst = out + big * big_bytes + ((static_cast<uint64_t>(iz) * B * bvy + iy * B) * bvx + ix * B) * eb +
-                       16u * k;
-        const int64_t y0 = static_cast<int64_t>(sy) * p.Beff - p.c, z0 = static_cast<int64_t>(sz) * p.Beff - p.c;
-        for (uint32_t r0 = 0; r0 < nrows; r0 += 4u) {
-            uint4 a[4], b[4];
+        // the slab's first byte in any row (negative in the covering left of x = 0)
+        const int64_t o0 = (static_cast<int64_t>(sx0) * p.Beff - p.c) * eb;
+        const int64_t y0 = static_cast<int64_t>(sy) * p.Beff - p.c;
+        const uint32_t lz0 = zp * sp.zlen, nz = min(sp.zlen, B - lz0);
+        const int64_t z0 = static_cast<int64_t>(sz) * p.Beff - p.c + lz0;  // of the block's first slice
+        const uint32_t nchunks = nbx * B * sp.cpr;
+        const uint32_t gy = sy / p.BB[1], gz = sz / p.BB[2];
+        uint8_t *const out0 = out + (static_cast<uint64_t>(gz) * p.nbig[1] + gy) * p.nbig[0] * big_bytes +
+                              (static_cast<uint64_t>((sz - gz * p.BB[2]) * B + lz0) * bvy + (sy - gy * p.BB[1]) * B) * drow;
+
+        // A thread's copies and chunks are the same in every slice up to the slice's
+        // offset: the first kPre of each are worked out once per slab.
+        struct Copy {
+            int64_t rb;    // the row's first byte in the level, in the block's first slice
+            uint32_t to;   // its place in a stage
+            uint32_t q;    // chunk of the row
+            bool in;       // the row lies inside the level's y range
+        };
+        auto copy_of = [&](uint32_t t) {
+            Copy c;
+            const uint32_t row = sp.by_cprow(t);
+            const int64_t y = y0 + row;
+            c.q = t - row * sp.cprow;
+            c.to = row * sp.pitch + 16u * c.q;
+            c.in = yz_vis && y >= 0 && y < p.D[1];
+            c.rb = z0 * plane + y * row_bytes;
+            return c;
+        };
+        auto copy_chunk = [&](const Copy &c, uint32_t i, uint32_t stage) {
+            const int64_t z = z0 + i, rb = c.rb + plane * i;
+            // inside the row from a chunk that reaches it on: the address is not negative
+            // there (the level is 16-byte aligned), and the cut copy ends at the row's end
+            int64_t a = ((rb + o0) & ~static_cast<int64_t>(15)) + 16 * static_cast<int64_t>(c.q);
+            const bool some = c.in && z >= 0 && z < p.D[2] && a + 16 > rb && a < rb + row_bytes;
+            const uint32_t n = some ? static_cast<uint32_t>(min(static_cast<int64_t>(16), rb + row_bytes - a)) : 0u;
+            copy16_async(stage + c.to, level + (some ? a : 0), n);
+        };
+        struct Chunk {
+            uint8_t *dst;     // in the block's first slice
+            uint32_t s;       // the row's offset in its first chunk, in the block's first slice
+            uint32_t row;     // the row's place in a stage
+            uint32_t at;      // the chunk's bytes after the row's offset
+            uint32_t zeros;   // leading zero bytes (the covering left of the row; all in an unvisited brick)
+        };
+        auto chunk_of = [&](uint32_t t) {
+            Chunk c;
+            const uint32_t j = sp.by_brick(t), r = t - j * (B * sp.cpr);
+            const uint32_t ly = sp.by_cpr(r), k = r - ly * sp.cpr;
+            const uint32_t sx = sx0 + j, gx = sx / p.BB[0];
+            c.dst = out0 + gx * big_bytes + ly * drow + (sx - gx * p.BB[0]) * B * eb + k * CH;
+            c.s = static_cast<uint32_t>(z0 * plane + (y0 + ly) * row_bytes + o0);
+            c.row = ly * sp.pitch;
+            c.at = j * p.Beff * eb + k * CH;
+            c.zeros = 0;
+            if (!yz_vis || static_cast<uint64_t>(sx) * p.Beff >= p.D[0])
+                c.zeros = CH;
+            else if (sx * p.Beff < p.c && k * CH < (p.c - sx * p.Beff) * eb)
+                c.zeros = (p.c - sx * p.Beff) * eb - k * CH;
+            return c;
+        };
+        // The chunk whose bytes start at byte `at` of the row `w`, to dst.
+        auto put_bytes = [&](const uint8_t *row, uint32_t at, uint32_t zeros, uint8_t *dst) {
+            const uint8_t *w = row + (at & ~static_cast<uint32_t>(CH - 1));
+            uint32_t v[CH / 4];
+            if constexpr (CH == 16) {
+                const uint4 x = window16(reinterpret_cast<const uint4 *>(w)[0], reinterpret_cast<const uint4 *>(w)[1],
+                                         at & 15u);
+                v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+            } else {
+                const uint2 x =
+                    window8(reinterpret_cast<const uint2 *>(w)[0], reinterpret_cast<const uint2 *>(w)[1], at & 7u);
+                v[0] = x.x, v[1] = x.y;
+            }
+            if (zeros) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint32_t r = r0 + u, ly = r & (B - 1u), lz = r >> p.b_shift;
-                const int64_t y = y0 + ly, z = z0 + lz;
-                const bool row_in = yz_vis && y >= 0 && z >= 0 && y < p.D[1] && z < p.D[2];
-                a[u] = make_uint4(0u, 0u, 0u, 0u);
-                b[u] = a[u];
-                if (row_in) {
-                    const uint4 *row = reinterpret_cast<const uint4 *>(
-                        level + (static_cast<uint64_t>(z) * p.D[1] + static_cast<uint64_t>(y)) * row_bytes);
-                    if (a_in) a[u] = __ldg(row + ca);
-                    if (b_in) b[u] = __ldg(row + ca + 1);
+                for (uint32_t q = 0; q < CH / 4; ++q) {
+                    const uint32_t z = zeros > 4u * q ? zeros - 4u * q : 0u;
+                    v[q] = z >= 4u ? 0u : v[q] & (0xffffffffu << (8u * z));
                 }
             }
-            if (valid) {
+            if constexpr (CH == 16)
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(v[0], v[1], v[2], v[3]);
+            else
+                *reinterpret_cast<uint2 *>(dst) = make_uint2(v[0], v[1]);
+        };
+        const uint64_t dslice = static_cast<uint64_t>(bvy) * drow;  // output slice stride
+        auto put_chunk = [&](const Chunk &c, uint32_t i, const uint8_t *stage) {
+            put_bytes(stage + c.row, ((c.s + static_cast<uint32_t>(plane) * i) & 15u) + c.at, c.zeros, c.dst + i * dslice);
+        };
+        constexpr uint32_t kPre = 2;
+        Copy cp[kPre];
+        Chunk ck[kPre];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const uint32_t r = r0 + u, ly = r & (B - 1u), lz = r >> p.b_shift;
-                    *reinterpret_cast<uint4 *>(dst + (static_cast<uint64_t>(lz) * bvy + ly) * drow) =
-                        window16(a[u], b[u], s);
+        for (uint32_t u = 0; u < kPre; ++u) {
+            cp[u] = copy_of(min(tid + 256u * u, ncopy - 1u));
+            ck[u] = chunk_of(min(tid + 256u * u, nchunks - 1u));
+        }
+        if ((plane & 15) == 0 && ncopy <= 256u * kPre && nchunks <= 256u * kPre) {
+            // Planes whole 16-byte chunks apart: a row starts at the same byte of its
+            // first chunk in every slice, so a thread's copies and chunks only advance
+            // by a plane and an output slice.
+            const uint8_t *src[kPre];
+            uint32_t n[kPre];
+#pragma unroll
+            for (uint32_t u = 0; u < kPre; ++u) {
+                const int64_t a = ((cp[u].rb + o0) & ~static_cast<int64_t>(15)) + 16 * static_cast<int64_t>(cp[u].q);
+                const bool some = cp[u].in && a + 16 > cp[u].rb && a < cp[u].rb + row_bytes;
+                n[u] = some ? static_cast<uint32_t>(min(static_cast<int64_t>(16), cp[u].rb + row_bytes - a)) : 0u;
+                src[u] = level + a;  // read only in slices inside the level
+                ck[u].at += ck[u].s & 15u;
+            }
+            uint32_t to_stage = 0, from_stage = 0;
+            auto next = [&](uint32_t st) { return st + slice_bytes == sp.stages * slice_bytes ? 0u : st + slice_bytes; };
+            auto copy_slice = [&](uint32_t i) {
+                if (i < nz) {
+                    const bool z_in = z0 + i >= 0 && z0 + i < p.D[2];  // the same for the block
+#pragma unroll
+                    for (uint32_t u = 0; u < kPre; ++u) {
+                        if (tid + 256u * u < ncopy) {
+                            const uint32_t k = z_in ? n[u] : 0u;
+                            copy16_async(smem + to_stage + cp[u].to, k ? src[u] : level, k);
+                        }
+                        src[u] += plane;
+                    }
+                    to_stage = next(to_stage);
                 }
+                copies_commit();
+            };
+            for (uint32_t i = 0; i + 1 < sp.stages; ++i) copy_slice(i);
+            for (uint32_t i = 0; i < nz; ++i) {
+                copies_wait(sp.stages - 2u);
+                __syncthreads();  // slice i is here for all, and slice i - 1 has been read by all
+                copy_slice(i + sp.stages - 1u);
+#pragma unroll
+                for (uint32_t u = 0; u < kPre; ++u) {
+                    if (tid + 256u * u < nchunks)
+                        put_bytes(slab_smem + from_stage + ck[u].row, ck[u].at, ck[u].zeros, ck[u].dst);
+                    ck[u].dst += dslice;
+                }
+                from_stage = next(from_stage);
+            }
+        } else {
+            auto copy_slice = [&](uint32_t i) {
+                if (i < nz) {
+                    const uint32_t stage = smem + (i % sp.stages) * slice_bytes;
+#pragma unroll
+                    for (uint32_t u = 0; u < kPre; ++u)
+                        if (tid + 256u * u < ncopy) copy_chunk(cp[u], i, stage);
+                    for (uint32_t t = tid + 256u * kPre; t < ncopy; t += 256u) copy_chunk(copy_of(t), i, stage);
+                }
+                copies_commit();
+            };
+            for (uint32_t i = 0; i + 1 < sp.stages; ++i) copy_slice(i);
+            for (uint32_t i = 0; i < nz; ++i) {
+                copies_wait(sp.stages - 2u);
+                __syncthreads();
+                copy_slice(i + sp.stages - 1u);
+                const uint8_t *stage = slab_smem + (i % sp.stages) * slice_bytes;
+#pragma unroll
+                for (uint32_t u = 0; u < kPre; ++u)
+                    if (tid + 256u * u < nchunks) put_chunk(ck[u], i, stage);
+                for (uint32_t t = tid + 256u * kPre; t < nchunks; t += 256u) put_chunk(chunk_of(t), i, stage);
             }
         }
+        __syncthreads();  // the last slices have been read before the next slab's copies
     }
+}
+
+// Launches the slab bricker where it applies: brick rows of whole 16- or 8-byte
+// chunks, a 16-byte aligned level, a store aligned to the chunks, and at least two
+// slices in shared memory.
+static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickParams &p, cudaStream_t s) {
+    const uint32_t row = p.B * p.eb;
+    const uint32_t ch = row % 16 == 0 ? 16u : (row % 8 == 0 ? 8u : 0u);
+    if (!ch || reinterpret_cast<uintptr_t>(level) % 16 || reinterpret_cast<uintptr_t>(out) % ch) return false;
+    SlabParams sp;
+    sp.p = p;
+    sp.cpr = row / ch;
+    const uint32_t nsx = p.nbig[0] * p.BB[0];
+    // about 512 output chunks a slice (two per thread), at most 1 KiB of a row
+    sp.nb = std::max(1u, std::min(std::min(nsx, 512u / std::max(1u, p.B * sp.cpr)), 1024u / (p.Beff * p.eb)));
+    sp.ngx = (nsx + sp.nb - 1) / sp.nb;
+    const uint32_t span = (sp.nb - 1) * p.Beff * p.eb + row;
+    sp.cprow = (15u + span + 15u) / 16u;
+    // the lanes of a quarter warp read 16-byte words of rows a pitch apart: cpr
+    // words on from row to row modulo the 8 words of a bank line
+    uint32_t words = sp.cprow + 1u;
+    if (sp.cpr < 8u)
+        while (words % 8u != (ch == 16 ? sp.cpr : 1u) % 8u) ++words;
+    sp.pitch = words * 16u;
+    const uint32_t slice = p.B * sp.pitch;
+    sp.stages = std::min(4u, (96u << 10) / slice);
+    if (sp.stages < 2u) sp.stages = std::min(2u, (200u << 10) / slice);
+    if (sp.stages < 2u || p.B * sp.cprow >= 65536u) return false;
+    const uint64_t slabs = static_cast<uint64_t>(sp.ngx) * (p.nbig[1] * p.BB[1]) * (p.nbig[2] * p.BB[2]);
+    // at least four blocks per SM, as far as a slab has slices
+    const uint64_t want = static_cast<uint64_t>(sm_count()) * 4u;
+    uint32_t parts = 1;
+    while (parts < p.B && slabs * parts < want) parts *= 2u;
+    sp.zlen = (p.B + parts - 1) / parts;
+    sp.zparts = (p.B + sp.zlen - 1) / sp.zlen;
+    sp.items = slabs * sp.zparts;
+    sp.by_cprow = SmallDiv(sp.cprow);
+    sp.by_brick = SmallDiv(p.B * sp.cpr);
+    sp.by_cpr = SmallDiv(sp.cpr);
+    const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(sp.items, 1u << 30));
+    const uint32_t bytes = sp.stages * slice;
+    auto go = [&](auto kernel) {
+        if (bytes > (48u << 10))
+            GC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+        kernel<<<grid, 256, bytes, s>>>(level, out, sp);
+    };
+    if (ch == 16)
+        go(brick_slab_kernel<16>);
+    else
+        go(brick_slab_kernel<8>);
+    GC_CUDA(cudaGetLastError());
+    count_launch();
+    return true;
 }
 
 // Bricks cut on demand from a device-resident pyramid (the device-levels
@@ -614,19 +850,8 @@ int gc_bricks_build(const void *level, const uint32_t level_dims[3], const gc_vo
         p.b_shift = p.cpr_shift = 0;
         while ((1u << p.b_shift) < p.B) ++p.b_shift;
         while (p.fast && (16u << p.cpr_shift) < p.B * p.eb) ++p.cpr_shift;
-        if (p.fast && p.cpr_shift <= 5) {
-            // runs of 32 / cpr bricks along x, one warp per run and brick row
-            const uint32_t nb = 32u >> p.cpr_shift;
-            const uint32_t ngx = (p.nbig[0] * p.BB[0] + nb - 1) / nb;
-            const uint64_t nseg = static_cast<uint64_t>(ngx) * (p.nbig[1] * p.BB[1]) * (p.nbig[2] * p.BB[2]);
-            const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((nseg + 7) / 8,
-                                                                           static_cast<uint64_t>(sm_count()) * 8));
-            brick_rows_kernel<<<static_cast<unsigned>(grid), 256, 0, as_stream(stream)>>>(
-                static_cast<const uint8_t *>(level), static_cast<uint8_t *>(out), p, ngx);
-            GC_CUDA(cudaGetLastError());
-            count_launch();
+        if (launch_brick_slabs(static_cast<const uint8_t *>(level), static_cast<uint8_t *>(out), p, as_stream(stream)))
             return;
-        }
         // one warp per brick: 8 warps per block, enough blocks to fill every SM
         const uint64_t grid = std::max<uint64_t>(1, std::min<uint64_t>((p.nsmall + 7) / 8,
                                                                        static_cast<uint64_t>(sm_count()) * 8));
