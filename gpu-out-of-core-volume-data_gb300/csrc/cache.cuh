@@ -176,28 +176,47 @@ struct CutSources {
 void launch_cut_bricks(const CutSources &srcs, const uint4 *jobs, uint32_t n, uint8_t *staging, uint64_t stride,
                        cudaStream_t s);
 
-// Scan control block shared by the decoupled look-back kernels.
+// Control block of the scans: zero between launches but for err (sticky) and
+// total.
 struct ScanCtl {
     uint32_t ticket;
     uint32_t done;
     uint32_t err;
-    uint32_t total;     // result: flagged items of the last scan
+    uint32_t total;     // result: flagged items of the last request scan
+    uint32_t used[2];   // running counts of a launch: used slots of the brick pool and the table pool
+    uint32_t pad[2];
 };
 
-constexpr uint32_t kErrLookback = 1u;   // a look-back wait ran out
+constexpr uint32_t kErrLookback = 1u;   // a wait for a predecessor's count ran out
 constexpr uint32_t kErrRender = 2u;     // render work-queue wait ran out
 
+// The scans of one frame (frame_scan_kernel): the request scan (nscan > 0) and
+// the used slots of one or two pools.
+struct FrameScan {
+    const uint32_t *req;
+    uint64_t nscan;            // entries scanned (0: no request scan)
+    uint32_t ts, maxreq;
+    uint4 *list;               // first maxreq flagged entries, decoded (device)
+    uint4 *host_list;          // and in pinned host memory, or null
+    uint32_t *host_total;      // pinned host memory: flagged entries, or null
+    uint32_t *out_total;       // a caller's result word on the device, or null
+    uint32_t mx, my;
+    const uint32_t *usage[2];
+    uint32_t nslots[2];        // 0: not counted
+    uint32_t *count[2];        // results (device)
+    uint64_t *status;          // a word per scan tile, zero between launches
+    ScanCtl *ctl;
+    uint32_t silent_tile;      // a tile that publishes nothing (tests of the error path; 0xffffffff: none)
+    uint32_t scan_tiles, count_blocks[2];  // set by launch_frame_scan
+};
+
 // Host launchers (cache_kernels.cu).
-void launch_lru_count(const uint32_t *usage, uint32_t nslots, uint32_t ts, uint32_t *count, cudaStream_t s);
+void launch_frame_scan(FrameScan a, const LevelTables &lt, cudaStream_t s);
 void launch_lru_partition(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
-                          uint32_t nslots, const uint32_t *count, uint64_t *status, ScanCtl *ctl,
-                          uint32_t epoch, cudaStream_t s);
-// silent_tile: a scan tile that publishes nothing (tests of the bounded
-// look-back's error path; 0xffffffff = none).
-void launch_miss_compact(const uint32_t *req, uint64_t nscan, uint32_t ts, uint32_t maxreq, uint4 *list,
-                         const LevelTables &lt, uint32_t mx, uint32_t my, uint64_t *status, ScanCtl *ctl,
-                         uint32_t epoch, cudaStream_t s, uint32_t silent_tile = 0xffffffffu);
-uint32_t lookback_tiles(uint64_t n);
+                          uint32_t nslots, const uint32_t *count, uint64_t *status, ScanCtl *ctl, cudaStream_t s);
+// Status words of the two kernels for n items.
+uint32_t lru_tiles(uint64_t n);
+uint32_t scan_tiles(uint64_t n);
 
 struct InstallArgs {
     uint4 *mrpd;

@@ -7,19 +7,20 @@
 // device_vector (CacheDevice.hpp:200-219): a stable partition, used slots
 // first.  That is one stable 1-bit radix pass on the key "used this frame"
 // (usage[slot] == timestamp).  Here the order is a list of 4-byte slot ids:
-//   lru_count      : total_used = #slots with usage == ts (one read of usage)
+//   frame_scan     : total_used = #slots with usage == ts (one read of usage)
 //   lru_partition  : per 4096-item tile, ballot/popc + block scan of the used
-//                    flags, decoupled look-back for the tile's exclusive
-//                    prefix P, then used id -> out[P + rank], unused id at
-//                    global index i -> out[total_used + i - used_before(i)].
+//                    flags, the tile's exclusive prefix P from the counts its
+//                    predecessors published, then used id -> out[P + rank],
+//                    unused id at global index i -> out[total_used + i -
+//                    used_before(i)].
 // Miss list.  The reference compacts indexes i in [0, size - 1) with
 // req[i] == ts with thrust::copy_if over a counting iterator into a full-size
 // size_t vector, keeps the first 50 and decodes them with coord_1D_to_3D
-// (CacheManager.hpp:409-474, CacheManagerKernels.cu:32-72).  miss_compact
-// does the scan, cap and decode in one pass with the same look-back scan.
-// Every look-back wait is bounded; on expiry the kernel sets ScanCtl::err.
+// (CacheManager.hpp:409-474, CacheManagerKernels.cu:32-72).  frame_scan does
+// the scan, cap and decode in one pass of its own blocks.
+// Every wait for a predecessor's count is bounded; on expiry the kernel sets
+// ScanCtl::err.
 #include <algorithm>
-#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -31,110 +32,70 @@
 namespace gc {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 16;
-constexpr uint32_t kTile = kThreads * kItems;
+constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kMaxSpins = 1u << 22;
+// lru_partition: 16 slot ids a lane; frame_scan: eight 16-byte words a lane
+constexpr uint32_t kLruItems = 16, kLruTile = kThreads * kLruItems;
+constexpr uint32_t kScanWords = 8, kScanTile = kThreads * kScanWords * 4;
 
-__device__ __forceinline__ void st_release(uint64_t *p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// A tile's status word: the published bit, then its count.  The word is all that
+// is handed over, so relaxed accesses do (no other memory is ordered by it).
+constexpr uint64_t kPublished = 1ull << 32;
+__device__ __forceinline__ void publish(uint64_t *status, uint32_t count) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(status), "l"(kPublished | count) : "memory");
 }
-__device__ __forceinline__ uint64_t ld_acquire(const uint64_t *p) {
+__device__ __forceinline__ uint64_t status_of(const uint64_t *status) {
     uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(status) : "memory");
     return v;
 }
 
-// Exclusive scan of one value per thread over a 256-thread block.
-__device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t &total) {
-    __shared__ uint32_t warp_tot[kThreads / 32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= static_cast<uint32_t>(o)) x += y;
-    }
-    if (lane == 31) warp_tot[warp] = x;
+// Sum of one value per thread over a block, for all threads.
+__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *s_warp) {
+    v = __reduce_add_sync(0xffffffffu, v);
     __syncthreads();
-    uint32_t pre = 0, tot = 0;
-#pragma unroll
-    for (uint32_t w = 0; w < kThreads / 32; ++w) {
-        const uint32_t t = warp_tot[w];
-        pre += (w < warp) ? t : 0u;
-        tot += t;
-    }
+    if ((threadIdx.x & 31u) == 0) s_warp[threadIdx.x >> 5] = v;
     __syncthreads();
-    total = tot;
-    return pre + x - v;
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) t += s_warp[w];
+    return t;
 }
 
-// Decoupled look-back (one warp).  Status word: [63:62] flag
-// (1 aggregate, 2 inclusive prefix), [61:32] launch epoch, [31:0] value.
-__device__ uint32_t lookback(uint64_t *status, uint32_t tile, uint32_t agg, uint32_t epoch, uint32_t *err,
-                             uint32_t silent_tile = 0xffffffffu) {
-    // Called by the 32 lanes of warp 0: each round reads the statuses of the
-    // 32 nearest unvisited predecessors at once (lane 0 the nearest) and sums
-    // the window up to the first inclusive prefix, waiting while a tile in
-    // that range has not published yet.  Returns the exclusive prefix (all
-    // lanes).  silent_tile (tests of the error path only) names a tile that
-    // publishes nothing, so that its successor's bounded wait runs out.
-    const uint32_t lane = threadIdx.x & 31u;
-    if (tile == silent_tile) return 0;
-    const uint32_t ep = epoch & 0x3FFFFFFFu;
-    const uint64_t E = static_cast<uint64_t>(ep) << 32;
-    if (tile == 0) {
-        if (lane == 0) st_release(&status[0], (2ull << 62) | E | agg);
-        return 0;
-    }
-    if (lane == 0) st_release(&status[tile], (1ull << 62) | E | agg);
-    uint32_t excl = 0;
-    int64_t top = static_cast<int64_t>(tile) - 1;
-    uint32_t spins = 0;
-    for (;;) {
-        const int64_t j = top - static_cast<int64_t>(lane);
-        uint64_t s = (2ull << 62) | E;  // before tile 0: an inclusive prefix of 0
-        if (j >= 0) s = ld_acquire(&status[j]);
-        const uint32_t flag = static_cast<uint32_t>(s >> 62);
-        const bool ready = (static_cast<uint32_t>(s >> 32) & 0x3FFFFFFFu) == ep && flag != 0;
-        const uint32_t incl = __ballot_sync(0xffffffffu, ready && flag == 2);
-        const uint32_t last = incl ? static_cast<uint32_t>(__ffs(incl)) - 1u : 31u;  // last lane needed
-        const uint32_t need = last == 31u ? 0xffffffffu : ((2u << last) - 1u);
-        if (__ballot_sync(0xffffffffu, !ready) & need) {
+// The number of flagged items in the tiles before `tile`, whose count this
+// tile's block has published: each thread waits (bounded) for the counts of
+// some predecessors, so that no tile waits for a chain of others.  Tiles are
+// handed out by a ticket, so every predecessor's block has started.
+__device__ uint32_t predecessors(const uint64_t *status, uint32_t tile, uint32_t *err, uint32_t *s_warp) {
+    uint32_t sum = 0, spins = 0;
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x; j < tile; j += kThreads) {
+        uint64_t v = status_of(status + j);
+        while (!(v & kPublished)) {
             if (++spins > kMaxSpins) {
-                if (lane == 0) atomicOr(err, kErrLookback);
+                atomicOr(err, kErrLookback);
                 break;
             }
-            __nanosleep(64);
-            continue;
+            __nanosleep(32);
+            v = status_of(status + j);
         }
-        excl += __reduce_add_sync(0xffffffffu, lane <= last ? static_cast<uint32_t>(s) : 0u);
-        if (incl) break;
-        top -= 32;
+        sum += static_cast<uint32_t>(v);
     }
-    if (lane == 0) st_release(&status[tile], (2ull << 62) | E | (excl + agg));
-    return excl;
+    return block_sum(sum, s_warp);
 }
 
-// The last block of a launch resets the ticket so the next launch needs no memset.
-__device__ __forceinline__ void finish_tile(ScanCtl *ctl) {
+// True in the block that ends a launch last: it leaves the tickets and status
+// words as the next launch expects them, with no memset between.
+__device__ __forceinline__ bool ends_launch(ScanCtl *ctl) {
+    __shared__ uint32_t s_last;
+    __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&ctl->done, 1u) == gridDim.x - 1) {
-            ctl->ticket = 0;
-            ctl->done = 0;
-            __threadfence();
-        }
+        s_last = atomicAdd(&ctl->done, 1u) == gridDim.x - 1u;
+        __threadfence();
     }
-}
-
-__global__ void __launch_bounds__(256) lru_count_kernel(const uint32_t *__restrict__ usage, uint32_t n,
-                                                        uint32_t ts, uint32_t *__restrict__ count) {
-    uint32_t c = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        c += (usage[i] == ts) ? 1u : 0u;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, c);
+    __syncthreads();
+    return s_last != 0;
 }
 
 __global__ void __launch_bounds__(kThreads) lru_partition_kernel(const uint32_t *__restrict__ order_in,
@@ -142,57 +103,58 @@ __global__ void __launch_bounds__(kThreads) lru_partition_kernel(const uint32_t 
                                                                  const uint32_t *__restrict__ usage,
                                                                  uint32_t ts, uint32_t n,
                                                                  const uint32_t *__restrict__ count,
-                                                                 uint64_t *status, ScanCtl *ctl,
-                                                                 uint32_t epoch) {
-    __shared__ uint32_t s_tile, s_excl;
+                                                                 uint64_t *status, ScanCtl *ctl) {
+    __shared__ uint32_t s_tile, s_warp[kWarps], s_used[kWarps];
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctl->ticket, 1u);
     __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint64_t base = static_cast<uint64_t>(tile) * kTile + threadIdx.x * kItems;
-    uint32_t ids[kItems];
-    uint32_t flags = 0;
+    const uint32_t tile = s_tile, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    // a warp's 512 consecutive items, 32 at a time
+    const uint64_t base = static_cast<uint64_t>(tile) * kLruTile + warp * (32u * kLruItems) + lane;
+    uint32_t ids[kLruItems], mine = 0, used = 0;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint64_t i = base + k;
-        ids[k] = 0;
-        if (i < n) {
-            ids[k] = order_in[i];
-            flags |= (usage[ids[k]] == ts ? 1u : 0u) << k;
-        }
-    }
-    uint32_t tile_total;
-    const uint32_t excl_thread = block_exclusive_scan(__popc(flags), tile_total);
-    if (threadIdx.x < 32) {
-        const uint32_t e = lookback(status, tile, tile_total, epoch, &ctl->err);
-        if (threadIdx.x == 0) s_excl = e;
-    }
+    for (uint32_t k = 0; k < kLruItems; ++k) ids[k] = base + 32u * k < n ? __ldg(order_in + base + 32u * k) : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kLruItems; ++k)
+        mine |= (base + 32u * k < n && usage[ids[k]] == ts ? 1u : 0u) << k;
+#pragma unroll
+    for (uint32_t k = 0; k < kLruItems; ++k) used += __popc(__ballot_sync(0xffffffffu, (mine >> k) & 1u));
+    if (lane == 0) s_used[warp] = used;
     __syncthreads();
+    uint32_t total = 0, before = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kWarps; ++w) {
+        before += w < warp ? s_used[w] : 0u;
+        total += s_used[w];
+    }
+    if (threadIdx.x == 0) publish(status + tile, total);
+    before += predecessors(status, tile, &ctl->err, s_warp);
     const uint32_t total_used = *count;
-    uint32_t used_before = s_excl + excl_thread;
     bool bad = false;
 #pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-        const uint64_t i = base + k;
+    for (uint32_t k = 0; k < kLruItems; ++k) {
+        const uint64_t i = base + 32u * k;
+        const uint32_t flags = __ballot_sync(0xffffffffu, (mine >> k) & 1u);
+        const uint32_t used_before = before + __popc(flags & ((1u << lane) - 1u));
         if (i < n) {
-            const uint64_t dst = ((flags >> k) & 1u) ? used_before
-                                                     : static_cast<uint64_t>(total_used) + i - used_before;
-            if ((flags >> k) & 1u) ++used_before;
+            const uint64_t dst = (mine >> k) & 1u ? used_before : total_used + i - used_before;
             if (dst < n)
                 order_out[dst] = ids[k];
             else
-                bad = true;  // only after a failed look-back
+                bad = true;  // only after an expired wait
         }
+        before += __popc(flags);
     }
     if (bad) atomicOr(&ctl->err, kErrLookback);
-    finish_tile(ctl);
+    if (ends_launch(ctl)) {
+        for (uint32_t j = threadIdx.x; j < gridDim.x; j += kThreads) status[j] = 0;
+        if (threadIdx.x == 0) ctl->ticket = ctl->done = 0;
+    }
 }
 
-__device__ __forceinline__ uint4 decode_request(uint64_t i, uint32_t mx, uint32_t my, const LevelTables &lt) {
-    const uint64_t xy = static_cast<uint64_t>(mx) * my;
-    const uint32_t z = static_cast<uint32_t>(i / xy);
-    const uint64_t r = i - static_cast<uint64_t>(z) * xy;
-    const uint32_t y = static_cast<uint32_t>(r / mx);
-    const uint32_t x = static_cast<uint32_t>(r - static_cast<uint64_t>(y) * mx);
+// coord_1D_to_3D (CacheManagerKernels.cu:32-72) of an entry (the page directory
+// has fewer than 2^32).
+__device__ __forceinline__ uint4 decode_request(uint32_t i, uint32_t mx, uint32_t my, const LevelTables &lt) {
+    const uint32_t row = i / mx, x = i - row * mx, z = row / my, y = row - z * my;
     uint32_t sum = 0, level = 0;
     for (level = 0; level < lt.nlevels; ++level) {
         sum += lt.nb[level][0];
@@ -202,47 +164,121 @@ __device__ __forceinline__ uint4 decode_request(uint64_t i, uint32_t mx, uint32_
     return make_uint4(x - (sum - lt.nb[level][0]), y, z, level);
 }
 
-__global__ void __launch_bounds__(kThreads) miss_compact_kernel(const uint32_t *__restrict__ req, uint64_t nscan,
-                                                                uint32_t ts, uint32_t maxreq,
-                                                                uint4 *__restrict__ list, const LevelTables lt,
-                                                                uint32_t mx, uint32_t my, uint64_t *status,
-                                                                ScanCtl *ctl, uint32_t epoch, uint32_t silent_tile) {
-    __shared__ uint32_t s_tile, s_excl;
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctl->ticket, 1u);
-    __syncthreads();
-    const uint32_t tile = s_tile;
-    const uint64_t base = static_cast<uint64_t>(tile) * kTile + threadIdx.x * kItems;
-    uint32_t flags = 0;
-    if (base + kItems <= nscan) {
-        const uint4 *p = reinterpret_cast<const uint4 *>(req + base);
+// The scans of a frame, each by blocks of its own: the request scan (scan_tiles
+// blocks) and the number of slots used (count_blocks[k] blocks for the brick
+// pool and the table pool of a two-level directory).  One launch, bound by the
+// read of the request buffer (from L2 when the frames follow one another).  A
+// request tile holds 8192 entries, eight 16-byte loads in flight a lane; it only
+// counts and publishes unless it has flagged entries, and then waits for its
+// predecessors' counts alone, not for a chain of them.  The miss list goes to the
+// device list and straight into the host's pinned copy: only the misses cross
+// the link, and no copy follows the scan.  6.4 M entries with 5000 misses: 29 us
+// (a chained look-back over 4096-entry tiles) -> 12 us.
+__global__ void __launch_bounds__(kThreads) frame_scan_kernel(const FrameScan a, const LevelTables lt) {
+    __shared__ uint32_t s_tile, s_warp[kWarps], s_used[kWarps];
+    __shared__ uint16_t s_entry[kScanTile];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (blockIdx.x < a.scan_tiles) {
+        if (threadIdx.x == 0) s_tile = atomicAdd(&a.ctl->ticket, 1u);
+        __syncthreads();
+        const uint32_t tile = s_tile;
+        // a warp's 1024 consecutive entries, 128 at a time
+        const uint64_t base = static_cast<uint64_t>(tile) * kScanTile + warp * (128u * kScanWords) + 4u * lane;
+        uint4 v[kScanWords];
+        uint32_t flags = 0;  // four bits a word
 #pragma unroll
-        for (int q = 0; q < kItems / 4; ++q) {
-            const uint4 v = __ldcs(p + q);
-            flags |= ((v.x == ts) ? 1u : 0u) << (4 * q);
-            flags |= ((v.y == ts) ? 1u : 0u) << (4 * q + 1);
-            flags |= ((v.z == ts) ? 1u : 0u) << (4 * q + 2);
-            flags |= ((v.w == ts) ? 1u : 0u) << (4 * q + 3);
+        for (uint32_t u = 0; u < kScanWords; ++u)
+            if (base + 128u * u + 4u <= a.nscan) v[u] = __ldcg(reinterpret_cast<const uint4 *>(a.req + base + 128u * u));
+#pragma unroll
+        for (uint32_t u = 0; u < kScanWords; ++u) {
+            const uint64_t i = base + 128u * u;
+            if (i + 4u <= a.nscan) {
+                flags |= ((v[u].x == a.ts ? 1u : 0u) | (v[u].y == a.ts ? 2u : 0u) | (v[u].z == a.ts ? 4u : 0u) |
+                          (v[u].w == a.ts ? 8u : 0u))
+                         << (4u * u);
+            } else {
+                for (uint32_t k = 0; k < 4u; ++k)
+                    if (i + k < a.nscan) flags |= (__ldcg(a.req + i + k) == a.ts ? 1u : 0u) << (4u * u + k);
+            }
+        }
+        const uint32_t used = __reduce_add_sync(0xffffffffu, __popc(flags));
+        if (lane == 0) s_used[warp] = used;
+        __syncthreads();
+        uint32_t total = 0, rank = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < kWarps; ++w) {
+            rank += w < warp ? s_used[w] : 0u;
+            total += s_used[w];
+        }
+        if (tile != a.silent_tile && tile < a.scan_tiles) {  // (beyond: calls that share the scratch overlapped)
+            if (threadIdx.x == 0) publish(a.status + tile, total);
+            if (total) {
+                // the tile's flagged entries in order, then decoded by all threads
+                for (uint32_t u = 0; u < kScanWords; ++u) {
+                    const uint32_t f = (flags >> (4u * u)) & 15u;
+                    if (!__any_sync(0xffffffffu, f)) continue;
+                    uint32_t r = rank;  // after the flagged entries of the lanes before
+#pragma unroll
+                    for (uint32_t k = 0; k < 4u; ++k) {
+                        const uint32_t bal = __ballot_sync(0xffffffffu, (f >> k) & 1u);
+                        r += __popc(bal & ((1u << lane) - 1u));
+                        rank += __popc(bal);
+                    }
+                    for (uint32_t k = 0; k < 4u; ++k)
+                        if ((f >> k) & 1u)
+                            s_entry[r++] = static_cast<uint16_t>(warp * (128u * kScanWords) + 128u * u + 4u * lane + k);
+                }
+                const uint32_t first = predecessors(a.status, tile, &a.ctl->err, s_warp);  // also a barrier
+                const uint32_t n = first < a.maxreq ? min(total, a.maxreq - first) : 0u;
+                for (uint32_t r = threadIdx.x; r < n; r += kThreads) {
+                    const uint4 b = decode_request(tile * kScanTile + s_entry[r], a.mx, a.my, lt);
+                    a.list[first + r] = b;
+                    if (a.host_list) a.host_list[first + r] = b;
+                }
+            }
         }
     } else {
-#pragma unroll
-        for (int k = 0; k < kItems; ++k)
-            if (base + k < nscan) flags |= ((req[base + k] == ts) ? 1u : 0u) << k;
+        uint32_t blk = blockIdx.x - a.scan_tiles;
+        const uint32_t k = blk < a.count_blocks[0] ? 0u : 1u;
+        if (k) blk -= a.count_blocks[0];
+        const uint32_t *__restrict__ usage = a.usage[k];
+        uint32_t c = 0;
+        for (uint32_t i = blk * kThreads + threadIdx.x; i < a.nslots[k]; i += a.count_blocks[k] * kThreads)
+            c += usage[i] == a.ts ? 1u : 0u;
+        c = block_sum(c, s_warp);
+        if (threadIdx.x == 0 && c) atomicAdd(&a.ctl->used[k], c);
     }
-    uint32_t tile_total;
-    const uint32_t excl_thread = block_exclusive_scan(__popc(flags), tile_total);
-    if (threadIdx.x < 32) {
-        const uint32_t e = lookback(status, tile, tile_total, epoch, &ctl->err, silent_tile);
-        if (threadIdx.x == 0) s_excl = e;
+    if (!ends_launch(a.ctl)) return;
+    // the last block: the totals, and everything as the next launch expects it
+    uint32_t sum = 0;
+    bool missing = false;
+    for (uint32_t j = threadIdx.x; j < a.scan_tiles; j += kThreads) {
+        const uint64_t v = status_of(a.status + j);
+        missing = missing || !(v & kPublished);
+        sum += static_cast<uint32_t>(v);
+        a.status[j] = 0;
     }
-    __syncthreads();
-    uint32_t rank = s_excl + excl_thread;
-    if (flags && rank < maxreq) {
-        for (int k = 0; k < kItems && rank < maxreq; ++k) {
-            if ((flags >> k) & 1u) list[rank++] = decode_request(base + k, mx, my, lt);
+    missing = __syncthreads_or(missing);
+    sum = block_sum(sum, s_warp);
+    if (threadIdx.x == 0) {
+        ScanCtl *ctl = a.ctl;
+        if (missing) ctl->err |= kErrLookback;
+        for (int k = 0; k < 2; ++k) {
+            if (a.count_blocks[k]) {
+                *a.count[k] = *static_cast<volatile uint32_t *>(&ctl->used[k]);
+                ctl->used[k] = 0;
+            }
         }
+        if (a.scan_tiles) {
+            ctl->total = sum;
+            if (a.host_total) *a.host_total = sum;
+            if (a.out_total) {  // a caller's own list: the result word tells a failure, and the next call starts clean
+                *a.out_total = *static_cast<volatile uint32_t *>(&ctl->err) ? GC_MISS_LIST_FAILED : sum;
+                ctl->err = 0;
+            }
+        }
+        ctl->ticket = ctl->done = 0;
     }
-    if (threadIdx.x == 0 && tile == gridDim.x - 1) ctl->total = s_excl + tile_total;
-    finish_tile(ctl);
 }
 
 // ---------------------------------------------------------------------------
@@ -730,30 +766,26 @@ __global__ void __launch_bounds__(256) completude_kernel(const float4 *__restric
 }
 
 // ---------------------------------------------------------------------------
-uint32_t lookback_tiles(uint64_t n) { return static_cast<uint32_t>(std::max<uint64_t>(1, (n + kTile - 1) / kTile)); }
+uint32_t lru_tiles(uint64_t n) { return static_cast<uint32_t>((n + kLruTile - 1) / kLruTile); }
+uint32_t scan_tiles(uint64_t n) { return static_cast<uint32_t>((n + kScanTile - 1) / kScanTile); }
 
-void launch_lru_count(const uint32_t *usage, uint32_t nslots, uint32_t ts, uint32_t *count, cudaStream_t s) {
-    GC_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t), s));
-    const uint32_t grid = std::min<uint32_t>(div_up(nslots, 256), static_cast<uint32_t>(sm_count()) * 4);
-    lru_count_kernel<<<std::max(1u, grid), 256, 0, s>>>(usage, nslots, ts, count);
+void launch_frame_scan(FrameScan a, const LevelTables &lt, cudaStream_t s) {
+    a.scan_tiles = a.nscan ? scan_tiles(a.nscan) : 0u;
+    uint32_t grid = a.scan_tiles;
+    for (int k = 0; k < 2; ++k) {
+        // a block per 4096 slots, at most two per SM
+        a.count_blocks[k] = a.nslots[k] ? std::min(div_up(a.nslots[k], 4096u), static_cast<uint32_t>(sm_count()) * 2u) : 0u;
+        grid += a.count_blocks[k];
+    }
+    frame_scan_kernel<<<grid, kThreads, 0, s>>>(a, lt);
     GC_CUDA(cudaGetLastError());
     count_launch();
 }
 
 void launch_lru_partition(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
-                          uint32_t nslots, const uint32_t *count, uint64_t *status, ScanCtl *ctl,
-                          uint32_t epoch, cudaStream_t s) {
-    lru_partition_kernel<<<lookback_tiles(nslots), kThreads, 0, s>>>(order_in, order_out, usage, ts, nslots,
-                                                                     count, status, ctl, epoch);
-    GC_CUDA(cudaGetLastError());
-    count_launch();
-}
-
-void launch_miss_compact(const uint32_t *req, uint64_t nscan, uint32_t ts, uint32_t maxreq, uint4 *list,
-                         const LevelTables &lt, uint32_t mx, uint32_t my, uint64_t *status, ScanCtl *ctl,
-                         uint32_t epoch, cudaStream_t s, uint32_t silent_tile) {
-    miss_compact_kernel<<<lookback_tiles(nscan), kThreads, 0, s>>>(req, nscan, ts, maxreq, list, lt, mx, my,
-                                                                   status, ctl, epoch, silent_tile);
+                          uint32_t nslots, const uint32_t *count, uint64_t *status, ScanCtl *ctl, cudaStream_t s) {
+    lru_partition_kernel<<<lru_tiles(nslots), kThreads, 0, s>>>(order_in, order_out, usage, ts, nslots, count, status,
+                                                                ctl);
     GC_CUDA(cudaGetLastError());
     count_launch();
 }
@@ -999,19 +1031,18 @@ void launch_completude(const float4 *slot_vpos, uint32_t nslots, uint32_t *count
 // frame deadline that must not block in the allocator (cudaMalloc can wait for
 // the device), or a plug-in whose host application owns every byte of device
 // memory and hands it only input and output buffers.  For them the scan's
-// scratch -- one look-back status word per 4096-entry tile and the scan
-// control block -- lives in this file-scope device array instead of memory
+// scratch -- one status word per 8192-entry tile and the scan control block -- lives in this file-scope device array instead of memory
 // obtained from cudaMalloc.  Every GPU that loads the library holds it until
 // the process exits.
 namespace gc {
 
-constexpr uint32_t kNoAllocMaxTiles = 2048;  // request buffers of up to 2048 * 4096 entries
-constexpr uint64_t kNoAllocMaxEntries = static_cast<uint64_t>(kNoAllocMaxTiles) * kTile;
+constexpr uint32_t kNoAllocMaxTiles = 1024;  // request buffers of up to 1024 * 8192 entries
+constexpr uint64_t kNoAllocMaxEntries = static_cast<uint64_t>(kNoAllocMaxTiles) * kScanTile;
 
-// words [0, kNoAllocMaxTiles): look-back status; the last two words: ScanCtl
+// ScanCtl, then a status word per tile
 constexpr uint32_t kNoAllocWords = kNoAllocMaxTiles + sizeof(ScanCtl) / sizeof(uint64_t);
-static_assert(sizeof(ScanCtl) == 2 * sizeof(uint64_t), "ScanCtl must fill two scratch words");
-static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];  // 16 KiB + 16 B
+static_assert(sizeof(ScanCtl) % sizeof(uint64_t) == 0, "ScanCtl must fill whole scratch words");
+static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];  // 8 KiB + 32 B
 
 // Host code cannot use g_noalloc_scratch as a device address (the name is a
 // host-side stand-in); the device address is looked up once per device, with
@@ -1019,13 +1050,6 @@ static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];  // 
 constexpr int kNoAllocMaxDevices = 64;
 static uint64_t *g_noalloc_ptr[kNoAllocMaxDevices] = {};
 static std::mutex g_noalloc_mu;
-
-// The scan's result word for the caller: the count of flagged entries, or
-// GC_MISS_LIST_FAILED when one of its bounded look-back waits ran out (the list
-// is then not valid).  Read on the device, so the call stays asynchronous.
-__global__ void noalloc_total_kernel(const ScanCtl *ctl, uint32_t *out_total) {
-    *out_total = ctl->err ? GC_MISS_LIST_FAILED : ctl->total;
-}
 
 // Test hook of the error path: GC_TEST_NOALLOC_SILENT_TILE=<k> makes scan tile
 // k publish nothing, so that tile k + 1's bounded look-back wait runs out.
@@ -1062,7 +1086,7 @@ extern "C" int gc_miss_list_noalloc(const uint32_t *requests, uint64_t n_entries
         GC_REQUIRE(n_entries >= 2, "the request buffer needs at least 2 entries");
         GC_REQUIRE(n_entries - 1 <= kNoAllocMaxEntries,
                    "request buffer too large for the allocation-free scan: at most 8388609 entries "
-                   "(2048 tiles of 4096) are supported");
+                   "(1024 tiles of 8192) are supported");
         GC_REQUIRE(max_requests >= 1, "max_requests must be >= 1");
         GC_REQUIRE(layout->nb_levels >= 1 && layout->nb_levels <= GC_MAX_LEVELS, "bad layout");
         // level tables of the page directory (levels packed along x)
@@ -1080,17 +1104,23 @@ extern "C" int gc_miss_list_noalloc(const uint32_t *requests, uint64_t n_entries
         GC_REQUIRE(static_cast<uint64_t>(mx) * my * mz == n_entries,
                    "n_entries does not match the page directory of the layout");
         cudaStream_t s = as_stream(stream);
-        uint64_t *status = noalloc_scratch();
-        ScanCtl *ctl = reinterpret_cast<ScanCtl *>(status + kNoAllocMaxTiles);
-        // The scratch keeps the previous call's contents: clear the control block
-        // and the status words this scan uses.
-        GC_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ScanCtl), s));
-        GC_CUDA(cudaMemsetAsync(status, 0, lookback_tiles(n_entries - 1) * sizeof(uint64_t), s));
-        static std::atomic<uint32_t> epoch{0};
-        launch_miss_compact(requests, n_entries - 1, timestamp, max_requests, reinterpret_cast<uint4 *>(out_list),
-                            lt, mx, my, status, ctl, epoch.fetch_add(1) + 1, s, noalloc_silent_tile());
-        noalloc_total_kernel<<<1, 1, 0, s>>>(ctl, out_total);
-        GC_CUDA(cudaGetLastError());
-        count_launch();
+        ScanCtl *ctl = reinterpret_cast<ScanCtl *>(noalloc_scratch());
+        uint64_t *status = reinterpret_cast<uint64_t *>(ctl + 1);
+        // The scan leaves the scratch as it found it, but calls that overlapped (see
+        // the header) may not have: every call starts from zeros.
+        GC_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ScanCtl) + scan_tiles(n_entries - 1) * sizeof(uint64_t), s));
+        FrameScan a{};
+        a.req = requests;
+        a.nscan = n_entries - 1;
+        a.ts = timestamp;
+        a.maxreq = max_requests;
+        a.list = reinterpret_cast<uint4 *>(out_list);
+        a.mx = mx;
+        a.my = my;
+        a.status = status;
+        a.ctl = ctl;
+        a.out_total = out_total;
+        a.silent_tile = noalloc_silent_tile();
+        launch_frame_scan(a, lt, s);
     });
 }

@@ -143,7 +143,7 @@ struct gc_cache {
     // two-level directory (d.pt_block > 0): directory words, table pool, its
     // LRU (ping-pong like the brick pool's) and the install's claim scratch
     gc::PageTable pt{};
-    uint32_t pt_slots = 0, pt_dims[3] = {0, 0, 0}, pt_cur = 0, epoch_pt = 0;
+    uint32_t pt_slots = 0, pt_dims[3] = {0, 0, 0}, pt_cur = 0;
     uint64_t pt_words = 0;
     uint32_t *pt_order[2] = {nullptr, nullptr};
     uint4 *pt_keys = nullptr;
@@ -182,7 +182,7 @@ struct gc_cache {
     cudaEvent_t ev_upload = nullptr, ev_upload_begin = nullptr;
     bool upload_timed = false;  // ev_upload_begin/ev_upload bracket an upload not yet counted
     int cur = 0;
-    uint32_t ts = 1, epoch_lru = 0, epoch_miss = 0;
+    uint32_t ts = 1;
     // loader
     bool gather = false;              // every host-store volume is read by the gather kernel
     bool vec16 = false;
@@ -551,18 +551,49 @@ static CacheView cache_view(const gc_cache *C) {
     return cv;
 }
 
-static void lru_update(gc_cache *C, cudaStream_t s) {
-    launch_lru_count(C->usage, C->nslots, C->ts, C->d_count, s);
+// The frame's scans and the LRU update; scan_slot >= 0: the request scan too, into
+// that miss list (its event marks the list and the count in host memory); mark:
+// flag the listed entries in flight (3).
+static void lru_update(gc_cache *C, cudaStream_t s, int scan_slot = -1, bool mark = false) {
+    FrameScan a{};
+    a.ts = C->ts;
+    a.status = C->status_miss;
+    a.ctl = C->ctl_miss;
+    a.silent_tile = 0xffffffffu;
+    a.usage[0] = C->usage;
+    a.nslots[0] = C->nslots;
+    a.count[0] = C->d_count;
+    if (C->pt.shift) {  // its counter word is pt_njobs, free between installs
+        a.usage[1] = C->pt.usage;
+        a.nslots[1] = C->pt_slots;
+        a.count[1] = C->pt_njobs;
+    }
+    if (scan_slot >= 0) {
+        gc_cache::MissList &L = C->lists[scan_slot];
+        a.req = C->req;
+        a.nscan = C->nentries - 1;
+        a.maxreq = C->d.max_requests;
+        a.list = L.d;
+        a.host_list = L.h;
+        a.host_total = L.total;
+        a.mx = C->mx;
+        a.my = C->my;
+    }
+    launch_frame_scan(a, C->lt, s);
+    if (scan_slot >= 0) {
+        gc_cache::MissList &L = C->lists[scan_slot];
+        if (mark)
+            launch_mark_in_flight(L.d, C->ctl_miss, C->d.max_requests, C->lt, C->mx, C->my, C->nentries, C->mrpd, s);
+        GC_CUDA(cudaEventRecord(L.ev, s));
+    }
     launch_lru_partition(C->order[C->cur], C->order[C->cur ^ 1], C->usage, C->ts, C->nslots, C->d_count,
-                         C->status_lru, C->ctl_lru, ++C->epoch_lru, s);
+                         C->status_lru, C->ctl_lru, s);
     C->cur ^= 1;
     if (C->pt.shift) {
         // the table pool's LRU (CacheManager::lru_update's loop over the
-        // table caches, CacheManager.hpp:386-406); its counter word is
-        // pt_njobs, free between installs
-        launch_lru_count(C->pt.usage, C->pt_slots, C->ts, C->pt_njobs, s);
+        // table caches, CacheManager.hpp:386-406)
         launch_lru_partition(C->pt_order[C->pt_cur], C->pt_order[C->pt_cur ^ 1], C->pt.usage, C->ts, C->pt_slots,
-                             C->pt_njobs, C->status_pt, C->ctl_pt, ++C->epoch_pt, s);
+                             C->pt_njobs, C->status_pt, C->ctl_pt, s);
         C->pt_cur ^= 1;
     }
 }
@@ -613,27 +644,16 @@ static void install(gc_cache *C, cudaStream_t s) {
     C->pend_nonempty = 0;
 }
 
-// Miss scan into list `slot`; mark: flag the listed entries in flight (3).
-static void scan_requests(gc_cache *C, cudaStream_t s, int slot = 0, bool mark = false) {
-    gc_cache::MissList &L = C->lists[slot];
-    launch_miss_compact(C->req, C->nentries - 1, C->ts, C->d.max_requests, L.d, C->lt, C->mx, C->my,
-                        C->status_miss, C->ctl_miss, ++C->epoch_miss, s);
-    if (mark) launch_mark_in_flight(L.d, C->ctl_miss, C->d.max_requests, C->lt, C->mx, C->my, C->nentries, C->mrpd, s);
-    GC_CUDA(cudaMemcpyAsync(L.h, L.d, C->d.max_requests * sizeof(uint4), cudaMemcpyDeviceToHost, s));
-    GC_CUDA(cudaMemcpyAsync(L.total, &C->ctl_miss->total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    GC_CUDA(cudaEventRecord(L.ev, s));
-}
-
 static bool update(gc_cache *C, cudaStream_t s) {
     GC_CUDA(cudaSetDevice(C->device));
-    lru_update(C, s);
     bool converged = false;
     if (C->sync_mode()) {
         if (C->done) {
+            lru_update(C, s);
             install(C, s);
             C->done = false;
         } else {
-            scan_requests(C, s);
+            lru_update(C, s, 0);
             C->cur_load = 0;  // the loader serves list 0 (an overlapped batch may have left 1)
             C->done = serve_request(C);
             converged = (C->stats.last_requests == 0);
@@ -641,23 +661,24 @@ static bool update(gc_cache *C, cudaStream_t s) {
     } else {
         std::unique_lock<std::mutex> lk(C->mu);
         if (!C->loader_error.empty()) {
+            lk.unlock();
+            lru_update(C, s);
+            lk.lock();
             std::string e = C->loader_error;
             C->loader_error.clear();
             fail(GC_ERR_IO, "brick loader: " + e);
         }
-        if (C->busy) {
-            C->ts++;
-            C->stats.frames++;
-            return false;
-        }
-        if (C->done) {
-            lk.unlock();
+        const bool busy = C->busy, done = C->done;
+        lk.unlock();
+        if (busy) {
+            lru_update(C, s);
+        } else if (done) {
+            lru_update(C, s);
             install(C, s);
             lk.lock();
             C->done = false;
         } else {
-            lk.unlock();
-            scan_requests(C, s);
+            lru_update(C, s, 0);
             C->cur_load = 0;  // the loader serves list 0 (an overlapped batch may have left 1)
             lk.lock();
             C->busy = true;
@@ -1036,13 +1057,13 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
             C->pt_word_of = dalloc<uint32_t>(maxr, "page-table claim words");
             C->pt_jobs = dalloc<uint2>(maxr, "page-table jobs");
             C->pt_njobs = dalloc<uint32_t>(1, "page-table job count");
-            C->status_pt = dalloc<uint64_t>(lookback_tiles(C->pt_slots), "scan status");
+            C->status_pt = dalloc<uint64_t>(lru_tiles(C->pt_slots), "scan status");
             C->ctl_pt = dalloc<ScanCtl>(1, "scan control");
             GC_CUDA(cudaMemset(C->pt.top, 0, C->pt_words * sizeof(uint32_t)));
             GC_CUDA(cudaMemset(C->pt.table, 0, C->pt_slots * per * sizeof(uint4)));
             GC_CUDA(cudaMemset(C->pt.usage, 0, C->pt_slots * sizeof(uint32_t)));
             GC_CUDA(cudaMemset(C->pt_claim, 0xff, C->pt_words * sizeof(uint32_t)));
-            GC_CUDA(cudaMemset(C->status_pt, 0, lookback_tiles(C->pt_slots) * sizeof(uint64_t)));
+            GC_CUDA(cudaMemset(C->status_pt, 0, lru_tiles(C->pt_slots) * sizeof(uint64_t)));
             GC_CUDA(cudaMemset(C->ctl_pt, 0, sizeof(ScanCtl)));
             launch_pt_init(C->pt_order[0], C->pt_keys, C->pt_slots, nullptr);
         } else {
@@ -1065,8 +1086,8 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
         C->d_samples = dalloc<unsigned long long>(2, "sample and ray counters");
         GC_CUDA(cudaMemset(C->d_samples, 0, 2 * sizeof(unsigned long long)));
         GC_CUDA(cudaMemset(C->slot_bins, 0xff, C->nslots * sizeof(unsigned long long)));
-        C->status_lru = dalloc<uint64_t>(lookback_tiles(C->nslots), "scan status");
-        C->status_miss = dalloc<uint64_t>(lookback_tiles(C->nentries), "scan status");
+        C->status_lru = dalloc<uint64_t>(lru_tiles(C->nslots), "scan status");
+        C->status_miss = dalloc<uint64_t>(scan_tiles(C->nentries), "scan status");
         C->ctl_lru = dalloc<ScanCtl>(1, "scan control");
         C->ctl_miss = dalloc<ScanCtl>(1, "scan control");
         C->d_count = dalloc<uint32_t>(1, "counter");
@@ -1097,8 +1118,8 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
         GC_CUDA(cudaMemset(C->req, 0, C->nentries * sizeof(uint32_t)));
         GC_CUDA(cudaMemset(C->usage, 0, C->nslots * sizeof(uint32_t)));
         GC_CUDA(cudaMemset(C->pool, 0, C->nslots * C->slot_bytes));
-        GC_CUDA(cudaMemset(C->status_lru, 0, lookback_tiles(C->nslots) * sizeof(uint64_t)));
-        GC_CUDA(cudaMemset(C->status_miss, 0, lookback_tiles(C->nentries) * sizeof(uint64_t)));
+        GC_CUDA(cudaMemset(C->status_lru, 0, lru_tiles(C->nslots) * sizeof(uint64_t)));
+        GC_CUDA(cudaMemset(C->status_miss, 0, scan_tiles(C->nentries) * sizeof(uint64_t)));
         GC_CUDA(cudaMemset(C->ctl_lru, 0, sizeof(ScanCtl)));
         GC_CUDA(cudaMemset(C->ctl_miss, 0, sizeof(ScanCtl)));
         GC_CUDA(cudaMemset(C->d_queue, 0, 4 * sizeof(uint32_t)));
@@ -1613,20 +1634,24 @@ static bool loader_idle(gc_cache *C) {
 // End of a rendered tick: LRU update and, with the loader idle, the scan.
 // Returns true when a scan was issued (its miss count lands in h_total).
 static bool batch_update(gc_cache *C, cudaStream_t s) {
-    lru_update(C, s);
     bool scanned = false;
     if (C->sync_mode()) {
-        if (!C->done) {
-            scan_requests(C, s);
+        if (C->done) {
+            lru_update(C, s);
+        } else {
+            lru_update(C, s, 0);
             C->cur_load = 0;  // the loader serves list 0 (an overlapped batch may have left 1)
             C->done = serve_request(C);
             scanned = true;
         }
     } else {
         std::unique_lock<std::mutex> lk(C->mu);
-        if (!C->busy && !C->done) {
+        if (C->busy || C->done) {
             lk.unlock();
-            scan_requests(C, s);
+            lru_update(C, s);
+        } else {
+            lk.unlock();
+            lru_update(C, s, 0);
             C->cur_load = 0;  // the loader serves list 0 (an overlapped batch may have left 1)
             lk.lock();
             C->busy = true;
@@ -1898,10 +1923,9 @@ static void batch_tick_overlapped(gc_batch *b, gc_cache *C, cudaStream_t s, uint
     render(C, views.data(), n, s, true, &b->graph, b->h_views);
     GC_CUDA(cudaEventRecord(b->ev_r1, s));
     GC_CUDA(cudaMemcpyAsync(b->h_status, b->d_status, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    lru_update(C, s);
+    // 4. the LRU update, and their requests into the free list, marked in flight
+    lru_update(C, s, free_slot, true);
     GC_CUDA(cudaMemcpyAsync(b->h_status + b->d.max_views, C->d_count, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    // 4. their requests into the free list, marked in flight
-    scan_requests(C, s, free_slot, true);
     const uint64_t serial = b->next_serial++;
     b->slot_state[free_slot] = 1;
     b->slot_serial[free_slot] = serial;

@@ -398,7 +398,7 @@ int gc_cache_last_misses(gc_cache_t cache, uint32_t *out4, uint32_t max, uint32_
  * scratch is a fixed array in device memory that every GPU loading the
  * library keeps until exit, so it suits callers that cannot allocate (stream
  * capture, hard frame deadlines, hosts that own all device memory).  Limits:
- * n_entries - 1 <= 8,388,608 (2048 scan tiles of 4096); larger buffers are
+ * n_entries - 1 <= 8,388,608 (1024 scan tiles of 8192); larger buffers are
  * rejected with GC_ERR_INVALID.  requests and out_list must be 16-byte
  * aligned and out_total 4-byte aligned (GC_ERR_INVALID otherwise, before any
  * device work).  The first call on a device looks the array's
