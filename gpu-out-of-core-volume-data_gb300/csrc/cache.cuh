@@ -292,22 +292,28 @@ struct RenderTuning {
     uint32_t precision = 0;  // 0: exact build (the oracle's operations); 1: fast build
 };
 RenderTuning &render_tuning();
+// What a ray-caster launch holds: one view with few or many rays, or several views.
+enum class MarchShape { kOneFew, kOneMany, kSeveral };
 // Ray-caster kernels of a voxel kind (1, 2, 4 bytes; 0 mixed widths; 0x202
 // two 8-bit channels) and brick size (16 and 32 have kernels
 // compiled for them; a two-level page directory has kernels of its own),
 // from the exact build (render.cu) or the fast build (render_fast.cu);
 // nullptr for an unsupported kind.
 namespace exact {
-void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, bool few_rays);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShape shape);
 }
 namespace fast {
-void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, bool few_rays);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShape shape);
 }
 // Fills ViewParams::visible of n device views from their transfer functions.
 void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s);
-void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev,
-                   const ViewParams *views_host, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
-                   uint32_t *queue, cudaStream_t s);
+void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev, uint32_t nviews,
+                   uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);
+// One view, its parameters in the launch; the visible bins are worked out by the
+// ray caster's blocks, for transfer functions of at most kOneViewTf entries.
+constexpr uint32_t kOneViewTf = 1024;
+void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewParams &view, uint32_t total_tiles,
+                       uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);
 
 // An executable CUDA graph of the batched launch (view-table copy + ray caster).
 struct RenderGraph {

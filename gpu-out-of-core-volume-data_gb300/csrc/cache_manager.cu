@@ -930,10 +930,14 @@ static void render(gc_cache *C, const gc_view *views, uint32_t n, cudaStream_t s
         launch_render_graph(*graph, cache_view(C), C->lt, C->d_views, pinned, n, tiles, rect_total, C->d_queue, s);
         return;
     }
+    if (n == 1 && vp[0].tfw <= kOneViewTf) {
+        launch_render_one(cache_view(C), C->lt, vp[0], tiles, rect_total, C->d_queue, s);
+        return;
+    }
     // pageable source: the call returns once the data is staged
     GC_CUDA(cudaMemcpyAsync(C->d_views, vp.data(), n * sizeof(ViewParams), cudaMemcpyHostToDevice, s));
     launch_view_bins(C->d_views, n, s);
-    launch_render(cache_view(C), C->lt, C->d_views, vp.data(), n, tiles, rect_total, C->d_queue, s);
+    launch_render(cache_view(C), C->lt, C->d_views, n, tiles, rect_total, C->d_queue, s);
 }
 
 // Upload route of the cache: the gather kernel when every volume with a host

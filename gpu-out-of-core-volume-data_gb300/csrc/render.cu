@@ -32,6 +32,7 @@
 #include "cache.cuh"
 #include "exact_math.cuh"
 #include "gc_internal.h"
+#include "view_bins.cuh"
 
 // The march below is compiled twice: here (namespace gc::exact, built with
 // -fmad=false: the oracle's operation sequence) and by render_fast.cu with
@@ -451,10 +452,9 @@ __device__ __forceinline__ uint4 load_entry(const CacheView &cv, const LevelTabl
 // (brick_below), else -1.
 template <bool TL>
 __device__ __forceinline__ int visit(const CacheView &cv, const LevelTables &lt, const ViewParams &vp, uint32_t lvl,
-                                     uint32_t lvl_end, V3 np, uint32_t idx, uint3 q, float max_op, Walk &w,
-                                     uint32_t &slvl) {
-    // read where used (rare paths): the view's visible bins (a newly entered
-    // brick) and its fallback flag (a missing one)
+                                     uint32_t lvl_end, V3 np, uint32_t idx, uint3 q, float max_op,
+                                     unsigned long long visible, Walk &w, uint32_t &slvl) {
+    // read where used (rare path): the view's fallback flag (a missing brick)
     if (idx != w.pidx) {
         // A new entry: the entry and its value bins are read together (one
         // memory round trip); the usage stamp of a mapped brick is a plain
@@ -463,7 +463,7 @@ __device__ __forceinline__ int visit(const CacheView &cv, const LevelTables &lt,
         const unsigned long long bins = __ldg(cv.entry_bins + idx);
         w.pidx = idx;
         w.flag = e.w;
-        w.invisible = (bins & vp.visible) == 0ull && (e.w == 1u || (e.w == 0u && cv.bins_user));
+        w.invisible = (bins & visible) == 0ull && (e.w == 1u || (e.w == 0u && cv.bins_user));
         if (e.w == 1u) {
             w.invisible = w.invisible || brick_below(bins, max_op);
             const uint32_t B = cv.B;
@@ -711,8 +711,11 @@ __device__ __forceinline__ float run_bound(const LevelTables &lt, const Ray &r, 
 
 // Returns false when the ray ended.  Else the ray stands at a sample (r.pend),
 // or it stepped through an invisible or empty brick.
-template <bool TL>
-__device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables &lt, Ray &r) {
+// ONE: the view's visible bins are kept in shared memory (`visible`), else in
+// its parameters.
+template <bool TL, bool ONE>
+__device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables &lt, const unsigned long long *visible,
+                                         Ray &r) {
     const ViewParams &vp = *r.vp;
     if (!((!r.dvr || r.fc.w < r.early) && r.t < r.tfar)) return false;
     const V3 np = norm_pos(r.pos);
@@ -743,8 +746,8 @@ __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables 
     V3 p;
     uint3 q;
     const uint32_t idx = entry_index(cv, lt, r.lvl, np, p, q);
-    const int st = visit<TL>(cv, lt, vp, r.lvl, r.lvl_end, np, idx, q, vp.skip_max ? r.maxOp : -1.0f, r.w,
-                             r.slvl);
+    const int st = visit<TL>(cv, lt, vp, r.lvl, r.lvl_end, np, idx, q, vp.skip_max ? r.maxOp : -1.0f,
+                             ONE ? *visible : vp.visible, r.w, r.slvl);
     if (st == kUnmapped) {
         vp.tbuf[r.i] = r.t;
         if (r.dvr)
@@ -882,10 +885,11 @@ __device__ __forceinline__ void ray_sample(const CacheView &cv, const LevelTable
 // One round of a warp's rays: the lanes that must find their next brick walk,
 // then the lanes that stand at a sample take it.  Returns true when the lane's
 // ray ended.
-template <typename T, uint32_t BS, bool TL, int N>
-__device__ __forceinline__ bool ray_round(const CacheView &cv, const LevelTables &lt, Ray &r, bool active) {
+template <typename T, uint32_t BS, bool TL, int N, bool ONE>
+__device__ __forceinline__ bool ray_round(const CacheView &cv, const LevelTables &lt,
+                                          const unsigned long long *visible, Ray &r, bool active) {
     bool ended = false;
-    if (active && !r.pend) ended = !ray_walk<TL>(cv, lt, r);
+    if (active && !r.pend) ended = !ray_walk<TL, ONE>(cv, lt, visible, r);
     __syncwarp();
     if (active && r.pend) ray_sample<T, BS, N>(cv, lt, r);
     __syncwarp();
@@ -992,19 +996,31 @@ __device__ __forceinline__ void retire_warp(uint32_t *queue, uint32_t nwarps) {
 // resident warps per SM) for launches of many rays, bound by issue; N = 4 with
 // all the registers it needs for launches of few rays, bound by latency
 // (render_launch_config).
+// ONE: a launch of one view, whose parameters come with the launch (`one`: no
+// table upload, read from constant memory) and whose visible bins each block
+// works out for itself (no kernel before this one).  The first tile of a warp is
+// its own number and a launch whose tiles all are first tiles never touches the
+// queue.  A 128^2 frame: 99 -> 93 us; 777x555, two channels: 2.14 -> 2.05 ms.
 constexpr uint32_t kWideWarps = 24;
-template <typename T, uint32_t BS, bool TL, int N>
+template <typename T, uint32_t BS, bool TL, int N, bool ONE>
 __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
-    render_kernel(const CacheView cv, const LevelTables lt, const ViewParams *__restrict__ views, uint32_t nviews,
-                  uint32_t total_tiles, uint32_t *queue, uint32_t nwarps) {
-    const uint32_t lane = threadIdx.x & 31u;
-    for (;;) {
-        uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(queue, 1u);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= total_tiles) break;
+    render_kernel(const CacheView cv, const LevelTables lt, const __grid_constant__ ViewParams one,
+                  const ViewParams *__restrict__ views, uint32_t nviews, uint32_t total_tiles, uint32_t *queue,
+                  uint32_t nwarps) {
+    __shared__ unsigned long long s_visible, s_samples[8], s_rays[8];  // of each warp
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0) s_samples[warp] = s_rays[warp] = 0;
+    if constexpr (ONE) {
+        if (threadIdx.x < 32u) {
+            const unsigned long long v = visible_bins(one, lane);
+            if (lane == 0) s_visible = v;
+        }
+        __syncthreads();
+    }
+    uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    while (t < total_tiles) {
         uint32_t tx, ty;
-        const ViewParams *vp = tile_of(views, nviews, t, tx, ty);
+        const ViewParams *vp = ONE ? tile_of(&one, 1u, t, tx, ty) : tile_of(views, nviews, t, tx, ty);
         const uint32_t sh = vp->tile_shift, tw = 1u << sh;
         const uint32_t x = (tx << sh) + (lane & (tw - 1u)), y = ty * (32u >> sh) + (lane >> sh);
         bool unm = false, coarse_any = false, marched = false;
@@ -1014,7 +1030,7 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
         bool active = x < vp->W && y < vp->H && ray_setup<T>(lt, vp, x, y, r);
         if (active) marched = ray_enters(r);
         while (__any_sync(0xffffffffu, active)) {
-            if (ray_round<T, BS, TL, N>(cv, lt, r, active)) {
+            if (ray_round<T, BS, TL, N, ONE>(cv, lt, &s_visible, r, active)) {
                 active = false;
                 unm = ray_finish(r);
                 coarse_any = r.coarse;
@@ -1023,42 +1039,53 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
         }
         const uint32_t tile_samples = __reduce_add_sync(0xffffffffu, nsamp);
         const uint32_t tile_rays = __popc(__ballot_sync(0xffffffffu, marched));
-        if (lane == 0 && tile_samples) atomicAdd(cv.samples, static_cast<unsigned long long>(tile_samples));
-        if (lane == 0 && tile_rays) atomicAdd(cv.samples + 1, static_cast<unsigned long long>(tile_rays));
+        if (lane == 0) {
+            s_samples[warp] += tile_samples;
+            s_rays[warp] += tile_rays;
+        }
         const uint32_t any = __ballot_sync(0xffffffffu, unm);
         if (any && lane == 0 && vp->status) atomicOr(vp->status, 1u);
         if (vp->fallback && vp->status) {  // bit 1: a coarser level stood in (preview image)
             const uint32_t coarse = __ballot_sync(0xffffffffu, coarse_any);
             if (coarse && lane == 0) atomicOr(vp->status, 2u);
         }
+        if (total_tiles <= nwarps) break;
+        if (lane == 0) t = nwarps + atomicAdd(queue, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0);
     }
-    retire_warp(queue, nwarps);
+    if (lane == 0 && s_samples[warp]) atomicAdd(cv.samples, s_samples[warp]);
+    if (lane == 0 && s_rays[warp]) atomicAdd(cv.samples + 1, s_rays[warp]);
+    if (total_tiles > nwarps) retire_warp(queue, nwarps);
 }
 
 // Kernel of a voxel kind (1, 2, 4 bytes, 0 mixed, kTwoChannelU8), brick size
 // (16 and 32 compiled for their size, others at run time) and samples at a
 // time; TL: for a two-level page directory.
-template <uint32_t BS, bool TL, int N>
+template <uint32_t BS, bool TL, int N, bool ONE>
 void *march_kernel_bs(uint32_t kind) {
     switch (kind) {
-        case 1: return reinterpret_cast<void *>(render_kernel<uint8_t, BS, TL, N>);
-        case 2: return reinterpret_cast<void *>(render_kernel<uint16_t, BS, TL, N>);
-        case 4: return reinterpret_cast<void *>(render_kernel<float, BS, TL, N>);
-        case 0: return reinterpret_cast<void *>(render_kernel<MixedVoxel, BS, TL, N>);
-        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N>);
+        case 1: return reinterpret_cast<void *>(render_kernel<uint8_t, BS, TL, N, ONE>);
+        case 2: return reinterpret_cast<void *>(render_kernel<uint16_t, BS, TL, N, ONE>);
+        case 4: return reinterpret_cast<void *>(render_kernel<float, BS, TL, N, ONE>);
+        case 0: return reinterpret_cast<void *>(render_kernel<MixedVoxel, BS, TL, N, ONE>);
+        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N, ONE>);
         default: return nullptr;
     }
 }
-template <int N>
+template <int N, bool ONE>
 void *march_kernel_n(uint32_t kind, uint32_t brick_size, bool two_level) {
     if (two_level)
-        return brick_size == 16 ? march_kernel_bs<16, true, N>(kind) : march_kernel_bs<0, true, N>(kind);
-    if (brick_size == 16) return march_kernel_bs<16, false, N>(kind);
-    if (brick_size == 32) return march_kernel_bs<32, false, N>(kind);
-    return march_kernel_bs<0, false, N>(kind);
+        return brick_size == 16 ? march_kernel_bs<16, true, N, ONE>(kind) : march_kernel_bs<0, true, N, ONE>(kind);
+    if (brick_size == 16) return march_kernel_bs<16, false, N, ONE>(kind);
+    if (brick_size == 32) return march_kernel_bs<32, false, N, ONE>(kind);
+    return march_kernel_bs<0, false, N, ONE>(kind);
 }
-void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, bool few_rays) {
-    return few_rays ? march_kernel_n<4>(kind, brick_size, two_level) : march_kernel_n<2>(kind, brick_size, two_level);
+void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShape shape) {
+    switch (shape) {
+        case MarchShape::kOneFew: return march_kernel_n<4, true>(kind, brick_size, two_level);
+        case MarchShape::kOneMany: return march_kernel_n<2, true>(kind, brick_size, two_level);
+        default: return march_kernel_n<2, false>(kind, brick_size, two_level);
+    }
 }
 
 }  // namespace GC_MARCH_NS
@@ -1127,38 +1154,12 @@ struct RenderLaunch {
     void *func;
     uint32_t grid, threads;
 };
-// Visible value bins of each view (empty-space skipping).  A sample whose
-// value lies in bin b reads transfer-function entries within
-// [floor(b/64 w - 1/2) - 1, floor((b+1)/64 w - 1/2) + 2]; its opacity after the
-// correction 1 - (1 - a)^k is below k a / (1 - a) <= 1.05 k a for a <= 0.04,
-// so with a the largest alpha of those entries and k the largest exponent of
-// the view's levels, a bin with 1.05 k a < 0.0009 never reaches the
-// compositing threshold 0.001.  One warp per view, two bins per lane.
+// Visible value bins of each view of a launch of several: one warp per view.
 __global__ void view_bins_kernel(ViewParams *views, uint32_t n) {
     const uint32_t v = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, lane = threadIdx.x & 31u;
     if (v >= n) return;
-    ViewParams &vp = views[v];
-    if (!vp.skip_empty) {
-        if (lane == 0) vp.visible = ~0ull;
-        return;
-    }
-    float kmax = 0.f;
-    for (uint32_t l = 0; l < vp.nlevels; ++l) kmax = fmaxf(kmax, vp.kexp[l]);
-    const int w = static_cast<int>(vp.tfw);
-    unsigned long long mine = 0;
-    for (uint32_t b = lane; b < kValueBins; b += 32) {
-        const float lo = static_cast<float>(b) / kValueBins, hi = static_cast<float>(b + 1) / kValueBins;
-        int i0 = static_cast<int>(floorf(lo * w - 0.5f)) - 1, i1 = static_cast<int>(floorf(hi * w - 0.5f)) + 2;
-        i0 = max(i0, 0);
-        i1 = min(i1, w - 1);
-        float amax = 0.f;
-        for (int i = i0; i <= i1; ++i) amax = fmaxf(amax, __ldg(vp.tf + 4 * i + 3));
-        const bool visible = !(amax <= 0.04f && 1.05f * kmax * amax < 0.0009f);
-        if (visible) mine |= 1ull << b;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0) vp.visible = mine;
+    const unsigned long long bins = visible_bins(views[v], lane);
+    if (lane == 0) views[v].visible = bins;
 }
 
 void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s) {
@@ -1173,7 +1174,7 @@ constexpr uint32_t kTwoChannelU8 = 0x202;
 static uint32_t voxel_kind(const CacheView &cv) { return cv.nc == 2 ? kTwoChannelU8 : cv.eb; }
 
 static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool two_level, uint32_t total_tiles,
-                                         uint32_t rect_tiles) {
+                                         uint32_t rect_tiles, bool one) {
     const RenderTuning tune = render_tuning();
     const uint32_t threads = tune.threads;
     GC_REQUIRE(threads == 64 || threads == 128 || threads == 256, "render threads must be 64, 128 or 256");
@@ -1187,15 +1188,17 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
     // samples at a time / 2): 464 such tiles 121 / 136 us, 1,950 tiles 336 / 408 us
     // a frame; 13,622 tiles 2.21 / 2.14 ms, 30,592 tiles 2.90 / 2.73 ms, 63,120
     // tiles 6.27 / 5.32 ms.
-    const bool few = rect_tiles <= static_cast<uint32_t>(sm_count()) * kWideWarps;
-    void *kernel = fast_build ? fast::march_kernel(eb, brick_size, two_level, few)
-                              : exact::march_kernel(eb, brick_size, two_level, few);
+    // Launches of several views take the shape for many rays.
+    const bool few = one && rect_tiles <= static_cast<uint32_t>(sm_count()) * kWideWarps;
+    const MarchShape shape = few ? MarchShape::kOneFew : (one ? MarchShape::kOneMany : MarchShape::kSeveral);
+    void *kernel = fast_build ? fast::march_kernel(eb, brick_size, two_level, shape)
+                              : exact::march_kernel(eb, brick_size, two_level, shape);
     if (!kernel) fail(GC_ERR_UNSUPPORTED, "the ray caster supports one channel of 1, 2 or 4 bytes");
     const int slot = eb == 1 ? 0 : eb == 2 ? 1 : eb == 4 ? 2 : eb == 0 ? 3 : 4;
-    static int occupancy[2][2][5][3][5] = {};
+    static int occupancy[2][3][5][3][5] = {};
     const int tslot = threads == 64 ? 0 : (threads == 128 ? 1 : 2);
     const int bslot = two_level ? (brick_size == 16 ? 3 : 4) : (brick_size == 16 ? 0 : (brick_size == 32 ? 1 : 2));
-    int &occ = occupancy[fast_build ? 1 : 0][few ? 1 : 0][slot][tslot][bslot];
+    int &occ = occupancy[fast_build ? 1 : 0][static_cast<int>(shape)][slot][tslot][bslot];
     if (!occ) {
         int b = 0;
         GC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kernel, static_cast<int>(threads), 0));
@@ -1208,14 +1211,26 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
     return RenderLaunch{kernel, std::max(1u, std::min(max_blocks, want)), threads};
 }
 
-void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev,
-                   const ViewParams * /*views_host*/, uint32_t nviews, uint32_t total_tiles,
-                   uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
+void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev, uint32_t nviews,
+                   uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.B, cv.pt.shift != 0u, total_tiles, rect_tiles);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.B, cv.pt.shift != 0u, total_tiles, rect_tiles, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
-    void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &views_dev, &nviews, &total_tiles,
-                    &queue, &nwarps};
+    ViewParams none{};
+    void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &none, &views_dev, &nviews,
+                    &total_tiles, &queue, &nwarps};
+    GC_CUDA(cudaLaunchKernel(L.func, dim3(L.grid), dim3(L.threads), args, 0, s));
+    count_launch();
+}
+
+void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewParams &view, uint32_t total_tiles,
+                       uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
+    if (total_tiles == 0) return;
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.B, cv.pt.shift != 0u, total_tiles, rect_tiles, true);
+    uint32_t nwarps = L.grid * (L.threads / 32), nviews = 1;
+    const ViewParams *views = nullptr;
+    void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), const_cast<ViewParams *>(&view),
+                    &views, &nviews, &total_tiles, &queue, &nwarps};
     GC_CUDA(cudaLaunchKernel(L.func, dim3(L.grid), dim3(L.threads), args, 0, s));
     count_launch();
 }
@@ -1240,10 +1255,11 @@ void launch_render_graph(RenderGraph &g, const CacheView &cv, const LevelTables 
                          const ViewParams *views_pinned, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
                          uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.B, cv.pt.shift != 0u, total_tiles, rect_tiles);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.B, cv.pt.shift != 0u, total_tiles, rect_tiles, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
     const ViewParams *vd = views_dev;
-    void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &vd, &nviews, &total_tiles,
+    ViewParams none{};
+    void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &none, &vd, &nviews, &total_tiles,
                     &queue, &nwarps};
     cudaKernelNodeParams kp = {};
     kp.func = L.func;

@@ -1,0 +1,40 @@
+// Visible value bins of a view (empty-space skipping), by one warp.
+#pragma once
+
+#include "cache.cuh"
+
+namespace gc {
+
+// A sample whose value lies in bin b reads transfer-function entries within
+// [floor(b/64 w - 1/2) - 1, floor((b+1)/64 w - 1/2) + 2]; its opacity after the
+// correction 1 - (1 - a)^k is below k a / (1 - a) <= 1.05 k a for a <= 0.04,
+// so with a the largest alpha of those entries and k the largest exponent of
+// the view's levels, a bin with 1.05 k a < 0.0009 never reaches the
+// compositing threshold 0.001.  Two bins per lane; every lane gets the result.
+// (Rounded operations throughout: the exact and the fast build agree.)
+__device__ __forceinline__ unsigned long long visible_bins(const ViewParams &vp, uint32_t lane) {
+    if (!vp.skip_empty) return ~0ull;
+    float kmax = 0.f;
+    for (uint32_t l = 0; l < vp.nlevels; ++l) kmax = fmaxf(kmax, vp.kexp[l]);
+    const int w = static_cast<int>(vp.tfw);
+    const float wf = static_cast<float>(w);
+    unsigned long long mine = 0;
+#pragma unroll
+    for (uint32_t b = lane; b < kValueBins; b += 32) {
+        const float lo = static_cast<float>(b) / kValueBins, hi = static_cast<float>(b + 1) / kValueBins;
+        int i0 = static_cast<int>(floorf(__fadd_rn(__fmul_rn(lo, wf), -0.5f))) - 1;
+        int i1 = static_cast<int>(floorf(__fadd_rn(__fmul_rn(hi, wf), -0.5f))) + 2;
+        i0 = max(i0, 0);
+        i1 = min(i1, w - 1);
+        float amax = 0.f;
+#pragma unroll 4
+        for (int i = i0; i <= i1; ++i) amax = fmaxf(amax, __ldg(vp.tf + 4 * i + 3));
+        const bool visible = !(amax <= 0.04f && __fmul_rn(__fmul_rn(1.05f, kmax), amax) < 0.0009f);
+        if (visible) mine |= 1ull << b;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mine |= __shfl_xor_sync(0xffffffffu, mine, o);
+    return mine;
+}
+
+}  // namespace gc

@@ -180,3 +180,43 @@ def test_launches_of_few_and_many_rays_agree(gc, torch_cuda, kind, mode, sampler
     assert any(x.any() for x in one)
     for x, y in zip(one, many):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("width", [1024, 1025])
+def test_visible_bins_of_either_launch_agree(gc, torch_cuda, width):
+    """A launch of one view works out its visible value bins itself up to 1024
+    transfer-function entries, from there on (and for several views) a kernel
+    before it does: bricks are skipped alike, so images, t, state and the number
+    of samples are the same."""
+    t = torch_cuda
+    n = 48
+    vol = gc.volume_desc((n, n, n), 8, 1, 1)
+    layout = gc.compute_layout(vol)
+    d = scenario.gpu_volume(gc, t, (n, n, n), 1, 9, 4)
+    store, offs, _ = gc.pre_process(vol, layout, d)
+    cm = gc.CacheManager(vol, layout, (11, 11, 11), max_requests=1000)
+    cm.set_source_host(store, offs)
+    tf = t.from_numpy(scenario.bumps_tf(5, width).reshape(-1)).cuda()
+    W, H = 60, 44
+    b = (t.zeros(W * H, dtype=t.int32, device="cuda"), t.zeros(W * H, device="cuda"), t.zeros(W * H * 4, device="cuda"))
+    view = gc.make_view(scenario.orbit_camera(gc, 2, 12, 2.4), W, H, tf.data_ptr(), width, b[0].data_ptr(),
+                        b[1].data_ptr(), b[2].data_ptr())
+    other = (t.zeros(1, dtype=t.int32, device="cuda"), t.zeros(1, device="cuda"), t.zeros(4, device="cuda"))
+    beside = gc.make_view(gc.look_at((0.0, 0.0, 9.0), (0.0, 0.0, 20.0)), 1, 1, tf.data_ptr(), width,
+                          other[0].data_ptr(), other[1].data_ptr(), other[2].data_ptr())  # looks away
+    for _ in range(60):
+        cm.render(view)
+        if cm.update():
+            break
+    got = []
+    for render in (lambda: cm.render(view), lambda: cm.render_batch([view, beside])):
+        for x in b:
+            x.zero_()
+        before = cm.stats()
+        render()
+        t.cuda.synchronize()
+        after = cm.stats()
+        got.append([x.cpu().numpy() for x in b] + [after.samples - before.samples, after.rays_marched - before.rays_marched])
+    for x, y in zip(*got):
+        assert np.array_equal(x, y)
+    assert got[0][3] > 0
