@@ -311,7 +311,7 @@ void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams 
                    uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);
 // One view, its parameters in the launch; the visible bins are worked out by the
 // ray caster's blocks, for transfer functions of at most kOneViewTf entries.
-constexpr uint32_t kOneViewTf = 1024;
+constexpr uint32_t kOneViewTf = 512;
 void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewParams &view, uint32_t total_tiles,
                        uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);
 
