@@ -140,8 +140,10 @@ def test_maximum_intensity_skips_change_nothing(gc, torch_cuda, bpc, sampler):
 @pytest.mark.parametrize("mode,sampler", [(0, 0), (0, 1), (1, 0), (1, 1)])
 def test_launches_of_few_and_many_rays_agree(gc, torch_cuda, kind, mode, sampler):
     """A launch of few rays takes more samples of a ray at a time than a launch of
-    many: the same views in launches of one view and of one batch (over 24 x 32
-    rays per SM) give the same image, t and colour state, bit for bit."""
+    many, and a launch of one view holds its transfer function in shared memory:
+    the same views in launches of one view, of one batch (over 24 x 32 rays per SM)
+    and of one batch with two tables give the same image, t and colour state, bit
+    for bit."""
     t = torch_cuda
     n, bpc, ch = 48, {"u16": 2, "f32": 4, "two": 2}.get(kind, 1), 2 if kind == "two" else 1
     B = 8 if kind == "u8_b8" else 16
@@ -179,9 +181,13 @@ def test_launches_of_few_and_many_rays_agree(gc, torch_cuda, kind, mode, sampler
 
     one = images(lambda: [cm.render(v) for v in views])
     many = images(lambda: cm.render_batch(views))
+    copy = tf_dev.clone()  # the views of this launch have different transfer functions
+    for v in views[1::2]:
+        v.tf = copy.data_ptr()
+    mixed = images(lambda: cm.render_batch(views))
     assert any(x.any() for x in one)
-    for x, y in zip(one, many):
-        assert np.array_equal(x, y)
+    for x, y, z in zip(one, many, mixed):
+        assert np.array_equal(x, y) and np.array_equal(x, z)
 
 
 @pytest.mark.parametrize("width", [1, 2, 256, 512, 513])
