@@ -172,9 +172,23 @@ struct CutSource {
 struct CutSources {
     CutSource vol[4];
 };
-// Cut jobs: {x, y, z, slot << 8 | volume << 6 | level} big bricks.
-void launch_cut_bricks(const CutSources &srcs, const uint4 *jobs, uint32_t n, uint8_t *staging, uint64_t stride,
-                       cudaStream_t s);
+// Where the bricks of each cache level come from, for loads that kernels resolve
+// from the miss list itself.
+struct StoreLevel {
+    uint64_t store;     // device address of the level's bricks in a host store, or 0
+    uint32_t nbx, nby;  // bricks per row, rows per slice
+    uint32_t bytes;     // of one brick
+    uint32_t cut;       // (volume << 6 | level) + 1 where bricks are cut from a device pyramid, else 0
+};
+struct StoreMap {
+    StoreLevel level[kMaxCacheLevels];
+};
+// Cut jobs: {x, y, z, slot << 8 | volume << 6 | level} big bricks, or (jobs null) a
+// miss list.
+void launch_cut_bricks(const CutSources &srcs, const uint4 *jobs, const uint4 *list, const StoreMap &m, uint32_t n,
+                       uint8_t *staging, uint64_t stride, cudaStream_t s);
+void launch_gather_missed(const uint4 *list, const StoreMap &m, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,
+                          cudaStream_t s);
 
 // Control block of the scans: zero between launches but for err (sticky) and
 // total.
@@ -246,7 +260,7 @@ struct InstallArgs {
     uint32_t *owner;           // per page-directory entry: lowest list index naming it (~0 between installs)
     uint64_t *coords;          // per list element: its page-directory entry
     const uint4 *asked;        // partitioned asked list: non-empty first
-    const uint32_t *big_index; // per non-empty brick
+    const uint32_t *big_index; // per non-empty brick; null: brick i is staged big brick i
     const uint4 *big_coord;    // per loaded big brick
     const uint8_t *staging;    // loaded big bricks
     uint32_t n, n_nonempty;

@@ -326,14 +326,12 @@ __device__ __forceinline__ float4 brick_origin(const LevelTables &lt, uint4 b, f
     return v;
 }
 
-// dereference_old_bricks (CacheManagerKernels.hpp:115-145) for the LRU tail.
-__global__ void install_evict_kernel(InstallArgs a, const LevelTables lt) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n_nonempty) return;
-    const uint32_t slot = a.order[a.nslots - a.n_nonempty + i];
+// dereference_old_bricks (CacheManagerKernels.hpp:115-145) for one slot of the
+// LRU tail, whose payload still names its old brick.
+__device__ __forceinline__ void evict_slot(const InstallArgs &a, const LevelTables &lt, uint32_t slot) {
     const float4 vp = a.slot_vpos[slot];
-    if (vp.x < 0.f) return;  // slot never held a brick
     const uint32_t level = a.slot_level[slot];
+    if (vp.x < 0.f) return;  // slot never held a brick
     const uint64_t e = mrpd_index(lt, level, vp.x, vp.y, vp.z, a.mx, a.my);
     if (e >= a.nentries) return;
     if (a.pt.shift) {
@@ -356,7 +354,7 @@ __global__ void install_evict_kernel(InstallArgs a, const LevelTables lt) {
 // Value range of a brick as value bins (empty-space skipping): min and max
 // over its voxels (covering included), normalized like the samplers, widened
 // by one bin on either side.  `at(v)` gives the address of voxel v; one
-// block per brick (up to 256 threads); the result is valid in thread 0.
+// block per brick (up to 288 threads); the result is valid in thread 0.
 // The value bins of the range [lo, hi] (normalized like the samplers), widened
 // by one bin on either side.
 __device__ __forceinline__ unsigned long long bins_of_range(float lo, float hi) {
@@ -376,7 +374,7 @@ __device__ unsigned long long block_bins_from(float lo, float hi) {
         lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
     }
-    __shared__ float s_lo[8], s_hi[8];
+    __shared__ float s_lo[9], s_hi[9];
     const uint32_t warp = threadIdx.x >> 5;
     if ((threadIdx.x & 31u) == 0) {
         s_lo[warp] = lo;
@@ -537,26 +535,45 @@ void launch_brick_bins(const uint8_t *level, const uint32_t nb[3], const uint32_
     count_launch();
 }
 
-// compute_lru_volume_position + copy_lru_position + write_brick
-// (CacheManagerKernels.cu:90-114, CacheManagerKernels.hpp:59-107): one block
-// per non-empty brick copies B^3 voxels from the staged big brick into the
-// LRU-tail slot, 16 bytes at a time when rows allow it.
-__global__ void __launch_bounds__(256) install_place_kernel(InstallArgs a, const LevelTables lt, float one_over_beff) {
+// One block per brick of the list, its first 256 threads copying and one more
+// warp keeping the books meanwhile, so that an install is two launches.
+//   books: dereference_old_bricks for the slot the brick takes, then the slot's
+//   new payload (compute_lru_volume_position + copy_lru_position,
+//   CacheManagerKernels.cu:90-114), and the owner word of the brick's entry (see
+//   install_reference_kernel);
+//   copy (write_brick, CacheManagerKernels.hpp:59-107): B^3 voxels from the staged
+//   big brick into the LRU-tail slot, 16 bytes at a time when rows allow it.
+// An evicted entry is read by nothing before install_reference_kernel.
+constexpr uint32_t kCopyThreads = 256;
+__global__ void __launch_bounds__(kCopyThreads + 32) install_place_kernel(InstallArgs a, const LevelTables lt,
+                                                                          float one_over_beff) {
     const uint32_t i = blockIdx.x;
-    if (i >= a.n_nonempty) return;
     const uint4 b = a.asked[i];
-    const uint32_t slot = a.order[a.nslots - a.n_nonempty + i];
-    if (threadIdx.x == 0) {
-        a.slot_level[slot] = b.w;
-        a.slot_vpos[slot] = brick_origin(lt, b, one_over_beff);
+    if (threadIdx.x == kCopyThreads) {
+        const float4 v = brick_origin(lt, b, one_over_beff);
+        const uint64_t c = mrpd_index(lt, b.w, v.x, v.y, v.z, a.mx, a.my);
+        a.coords[i] = c;
+        if (c < a.nentries) atomicMin(a.owner + c, i);
+        if (i < a.n_nonempty) {
+            const uint32_t slot = a.order[a.nslots - a.n_nonempty + i];
+            evict_slot(a, lt, slot);
+            a.slot_level[slot] = b.w;
+            a.slot_vpos[slot] = v;
+        }
     }
+    if (i >= a.n_nonempty) return;  // an empty brick: books only
+    const uint32_t slot = a.order[a.nslots - a.n_nonempty + i];
+    const uint32_t tid = threadIdx.x;  // the last warp copies nothing and only joins the block's barriers
     // the brick's volume: voxel width and big-brick shape of its level
     const uint32_t B = a.B, eb = lt.eb[b.w];
     const uint32_t *BB = lt.bb[b.w];
     const uint32_t bvx = BB[0] * B, bvy = BB[1] * B;
-    const uint32_t bi = a.big_index[i];
-    const uint4 bc = a.big_coord[bi];
-    const uint32_t ox = (b.x - bc.x * BB[0]) * B, oy = (b.y - bc.y * BB[1]) * B, oz = (b.z - bc.z * BB[2]) * B;
+    uint32_t bi = i, ox = 0, oy = 0, oz = 0;
+    if (a.big_index) {  // else every big brick is one brick, staged in list order
+        bi = a.big_index[i];
+        const uint4 bc = a.big_coord[bi];
+        ox = (b.x - bc.x * BB[0]) * B, oy = (b.y - bc.y * BB[1]) * B, oz = (b.z - bc.z * BB[2]) * B;
+    }
     const uint8_t *src = a.staging + bi * a.big_stride;
     uint8_t *dst = a.pool + static_cast<uint64_t>(slot) * a.slot_bytes;
     const uint32_t row_bytes = B * eb;
@@ -571,11 +588,11 @@ __global__ void __launch_bounds__(256) install_place_kernel(InstallArgs a, const
         const uint32_t nvec = rows * vec_per_row;
         const bool bins = a.slot_bins && a.nc == 1;
         float lo = 3.4e38f, hi = -3.4e38f;
-        for (uint32_t v0 = threadIdx.x; v0 < nvec; v0 += 4u * blockDim.x) {
+        for (uint32_t v0 = tid < kCopyThreads ? tid : nvec; v0 < nvec; v0 += 4u * kCopyThreads) {
             uint4 val[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const uint32_t v = v0 + u * blockDim.x;
+                const uint32_t v = v0 + u * kCopyThreads;
                 if (v < nvec) {
                     const uint32_t r = v >> qs, q = v & (vec_per_row - 1u);
                     const uint32_t ly = r & (B - 1u), lz = r >> bs;
@@ -586,7 +603,7 @@ __global__ void __launch_bounds__(256) install_place_kernel(InstallArgs a, const
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const uint32_t v = v0 + u * blockDim.x;
+                const uint32_t v = v0 + u * kCopyThreads;
                 if (v < nvec) {
                     reinterpret_cast<uint4 *>(dst)[v] = val[u];
                     if (bins) chunk_range(val[u], eb, lo, hi);
@@ -603,7 +620,7 @@ __global__ void __launch_bounds__(256) install_place_kernel(InstallArgs a, const
         return;
     } else {
         const uint32_t nbytes = rows * row_bytes;
-        for (uint32_t v = threadIdx.x; v < nbytes; v += blockDim.x) {
+        for (uint32_t v = tid < kCopyThreads ? tid : nbytes; v < nbytes; v += kCopyThreads) {
             const uint32_t r = v / row_bytes, q = v % row_bytes;
             const uint32_t ly = r % B, lz = r / B;
             const uint64_t soff = ((static_cast<uint64_t>(oz + lz) * bvy + (oy + ly)) * bvx + ox) * eb + q;
@@ -626,18 +643,8 @@ __global__ void __launch_bounds__(256) install_place_kernel(InstallArgs a, const
 // already mapped or empty is left alone.  The reference walks the list in one
 // thread; here each brick is one thread, and a brick whose MRPD entry also
 // belongs to an earlier list element yields to it, which is the serial order:
-// the first pass leaves the lowest list index naming each entry in `owner`,
-// the second lets only that element act (and puts the owner word back).
-__global__ void install_owner_kernel(InstallArgs a, const LevelTables lt, float one_over_beff) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.n) return;
-    const uint4 b = a.asked[i];
-    const float4 v = brick_origin(lt, b, one_over_beff);
-    const uint64_t c = mrpd_index(lt, b.w, v.x, v.y, v.z, a.mx, a.my);
-    a.coords[i] = c;
-    if (c < a.nentries) atomicMin(a.owner + c, i);
-}
-
+// install_place_kernel leaves the lowest list index naming each entry in `owner`,
+// and only that element acts (and puts the owner word back).
 __global__ void install_reference_kernel(InstallArgs a, const LevelTables lt, float one_over_beff) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.n) return;
@@ -826,15 +833,7 @@ void launch_live_bins(const LevelTables &lt, const float4 *slot_vpos, const uint
 void launch_install(const InstallArgs &a, const LevelTables &lt, cudaStream_t s) {
     if (a.n == 0) return;
     const float one_over_beff = 1.0f / static_cast<float>(a.Beff);
-    if (a.n_nonempty) {
-        install_evict_kernel<<<div_up(a.n_nonempty, 128), 128, 0, s>>>(a, lt);
-        GC_CUDA(cudaGetLastError());
-        count_launch();
-        install_place_kernel<<<a.n_nonempty, 256, 0, s>>>(a, lt, one_over_beff);
-        GC_CUDA(cudaGetLastError());
-        count_launch();
-    }
-    install_owner_kernel<<<div_up(a.n, 256u), 256, 0, s>>>(a, lt, one_over_beff);
+    install_place_kernel<<<a.n, kCopyThreads + 32, 0, s>>>(a, lt, one_over_beff);
     GC_CUDA(cudaGetLastError());
     count_launch();
     if (a.pt.shift) {
@@ -899,11 +898,27 @@ void launch_pt_init(uint32_t *order, uint4 *keys, uint32_t nslots, cudaStream_t 
 // writes land in the device staging buffer the install kernels read.
 // kIlp independent loads per thread are in flight before their stores: the
 // host link's latency (microseconds) needs many bytes in flight per SM.
-template <typename W, uint32_t kIlp>
-__device__ __forceinline__ void gather_bricks(const ulonglong2 *__restrict__ src, uint32_t n, uint64_t stride,
-                                              uint8_t *__restrict__ dst) {
+// src(b): brick b as {address, bytes}.
+struct ListedBricks {
+    const ulonglong2 *__restrict__ src;
+    __device__ __forceinline__ ulonglong2 operator()(uint32_t b) const { return src[b]; }
+};
+// Brick b of a miss list in the host stores of its volume (each big brick one
+// brick); nothing to read where the volume's source is not a host store.
+struct MissedBricks {
+    const uint4 *__restrict__ list;
+    const StoreMap &m;
+    __device__ __forceinline__ ulonglong2 operator()(uint32_t b) const {
+        const uint4 e = list[b];
+        const StoreLevel &l = m.level[e.w];
+        return make_ulonglong2(l.store + ((static_cast<uint64_t>(e.z) * l.nby + e.y) * l.nbx + e.x) * l.bytes,
+                               l.store ? l.bytes : 0u);
+    }
+};
+template <typename W, uint32_t kIlp, class Src>
+__device__ __forceinline__ void gather_bricks(const Src src, uint32_t n, uint64_t stride, uint8_t *__restrict__ dst) {
     for (uint32_t b = blockIdx.x; b < n; b += gridDim.x) {
-        const ulonglong2 e = src[b];  // {address, bytes}
+        const ulonglong2 e = src(b);
         const W *sp = reinterpret_cast<const W *>(e.x);
         W *dp = reinterpret_cast<W *>(dst + static_cast<uint64_t>(b) * stride);
         const uint64_t words = e.y / sizeof(W);
@@ -926,13 +941,30 @@ __device__ __forceinline__ void gather_bricks(const ulonglong2 *__restrict__ src
 template <typename W>
 __global__ void gather_bricks_kernel(const ulonglong2 *__restrict__ src, uint32_t n, uint64_t stride,
                                      uint8_t *__restrict__ dst) {
-    gather_bricks<W, 4>(src, n, stride, dst);
+    gather_bricks<W, 4>(ListedBricks{src}, n, stride, dst);
 }
 // At most 32 registers per thread (128 threads, 16 blocks): fits beside the ray caster.
 template <typename W>
 __global__ void __launch_bounds__(128, 16) gather_bricks_beside_kernel(const ulonglong2 *__restrict__ src, uint32_t n,
                                                                       uint64_t stride, uint8_t *__restrict__ dst) {
-    gather_bricks<W, 2>(src, n, stride, dst);
+    gather_bricks<W, 2>(ListedBricks{src}, n, stride, dst);
+}
+template <typename W>
+__global__ void __launch_bounds__(128, 16) gather_missed_kernel(const uint4 *__restrict__ list, const StoreMap m,
+                                                               uint32_t n, uint64_t stride, uint8_t *__restrict__ dst) {
+    gather_bricks<W, 2>(MissedBricks{list, m}, n, stride, dst);
+}
+
+void launch_gather_missed(const uint4 *list, const StoreMap &m, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,
+                          cudaStream_t s) {
+    if (n == 0) return;
+    const uint32_t grid = std::min<uint32_t>(n, static_cast<uint32_t>(sm_count()));  // as beside a render (below)
+    if (vec16)
+        gather_missed_kernel<uint4><<<grid, 128, 0, s>>>(list, m, n, stride, dst);
+    else
+        gather_missed_kernel<uint8_t><<<grid, 128, 0, s>>>(list, m, n, stride, dst);
+    GC_CUDA(cudaGetLastError());
+    count_launch();
 }
 
 void launch_gather_bricks(const ulonglong2 *src, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,

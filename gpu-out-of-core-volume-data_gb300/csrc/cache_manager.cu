@@ -191,6 +191,10 @@ struct gc_cache {
     std::condition_variable cv;
     bool stop = false, has_request = false, busy = false, done = false, last_converged = false;
     uint32_t pend_n = 0, pend_nonempty = 0;
+    const uint4 *pend_list = nullptr;  // the list to install where the device resolved it, else null (d_asked)
+    bool direct = false;              // loads are resolved on the device (update_upload_route)
+    bool direct_host = false, direct_cut = false;  // ... from host stores / from device pyramids
+    gc::StoreMap stores{};            // their sources
     std::string loader_error;
     gc_cache_stats stats;
 
@@ -259,10 +263,45 @@ static void build_tables(gc_cache *C) {
                         : 0u;
 }
 
+// A load that the device resolves: with one-brick big bricks, no empty bricks and
+// every volume in a host store that the device reads or in a device pyramid, the
+// miss list itself says what to copy where -- element i is staged big brick i.
+// The host only looks the elements over (one outside its level -- a caller's own
+// request buffer may flag the directory's padding -- takes the general route) and
+// nothing of the list is sent back to the device.  Returns false to take the
+// general route.
+static bool load_listed(gc_cache *C, uint32_t n, std::chrono::steady_clock::time_point t_begin) {
+    const gc_cache::MissList &L = C->lists[C->cur_load];
+    uint64_t bytes = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint4 b = L.h[i];
+        if (b.w >= C->lt.nlevels || b.x >= C->lt.nb[b.w][0] || b.y >= C->lt.nb[b.w][1] || b.z >= C->lt.nb[b.w][2])
+            return false;
+        if (C->stores.level[b.w].store) bytes += C->stores.level[b.w].bytes;
+    }
+    C->pend_n = C->pend_nonempty = n;
+    C->pend_list = L.d;
+    C->stats.load_cycles++;
+    C->stats.loader_host_ns += static_cast<uint64_t>(
+        std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t_begin).count());
+    // on the side stream, beside the next frame's render, as below; the scan that
+    // wrote the list has ended (its event was waited for)
+    cudaStream_t s = C->side;
+    GC_CUDA(cudaEventRecord(C->ev_upload_begin, s));
+    if (C->direct_host) launch_gather_missed(L.d, C->stores, n, C->big_stride, C->d_staging, C->vec16, s);
+    if (C->direct_cut) launch_cut_bricks(C->cut, nullptr, L.d, C->stores, n, C->d_staging, C->big_stride, s);
+    GC_CUDA(cudaEventRecord(C->ev_upload, s));
+    C->upload_timed = true;
+    C->stats.bytes_h2d += bytes;
+    C->stats.requests_served += n;
+    return true;
+}
+
 // Resolve the asked bricks: RequestHandler::handle_request (RequestHandler.hpp:277-372).
 // Returns the number of bricks to install (non-empty first), or 0.
 static void resolve_and_upload(gc_cache *C, uint32_t n) {
     const auto t_begin = std::chrono::steady_clock::now();
+    if (C->direct && load_listed(C, n, t_begin)) return;
     ResolveScratch &R = C->resolve;
     R.kind.assign(n, 0);  // 0 non-empty, 1 empty, 2 unknown (dropped)
     std::vector<int> &kind = R.kind;
@@ -437,6 +476,7 @@ static void resolve_and_upload(gc_cache *C, uint32_t n) {
     std::memcpy(C->h_big_index, big_index.data(), big_index.size() * sizeof(uint32_t));
     C->pend_n = k;
     C->pend_nonempty = n_nonempty;
+    C->pend_list = nullptr;
     C->stats.load_cycles++;
     C->stats.loader_host_ns += static_cast<uint64_t>(
         std::chrono::duration_cast<std::chrono::nanoseconds>(std::chrono::steady_clock::now() - t_begin).count());
@@ -459,7 +499,7 @@ static void resolve_and_upload(gc_cache *C, uint32_t n) {
     }
     if (ncut) {  // after the host bricks: a staged copy covers every slot
         GC_CUDA(cudaMemcpyAsync(C->d_cut, C->h_cut, ncut * sizeof(uint4), cudaMemcpyHostToDevice, s));
-        launch_cut_bricks(C->cut, C->d_cut, ncut, C->d_staging, C->big_stride, s);
+        launch_cut_bricks(C->cut, C->d_cut, nullptr, C->stores, ncut, C->d_staging, C->big_stride, s);
     }
     GC_CUDA(cudaMemcpyAsync(C->d_asked, C->h_asked, k * sizeof(uint4), cudaMemcpyHostToDevice, s));
     if (n_nonempty) {
@@ -629,10 +669,10 @@ static void install(gc_cache *C, cudaStream_t s) {
     a.entry_bins = C->entry_bins;
     a.user_bins = C->user_bins;
     a.nc = C->nc;
-    a.asked = C->d_asked;
+    a.asked = C->pend_list ? C->pend_list : C->d_asked;
     a.owner = C->d_owner;
     a.coords = C->d_coords;
-    a.big_index = C->d_big_index;
+    a.big_index = C->pend_list ? nullptr : C->d_big_index;
     a.big_coord = C->d_big_coord;
     a.staging = C->d_staging;
     a.n = C->pend_n;
@@ -955,6 +995,29 @@ static void update_upload_route(gc_cache *C) {
     }
     C->gather = any && all;
     C->vec16 = vec16;
+    // loads resolved on the device (load_listed)
+    C->direct = true;
+    C->direct_host = C->direct_cut = false;
+    std::memset(&C->stores, 0, sizeof(C->stores));
+    for (uint32_t v = 0; v < C->vols.size(); ++v) {
+        const Volume &V = C->vols[v];
+        const uint32_t *BB = V.desc.big_brick_size;
+        const bool host = V.src.kind == 1 && C->gather, cut = V.src.kind == 5;
+        if (!(host || cut) || BB[0] * BB[1] * BB[2] != 1u || !V.src.empty.empty() || V.big_bytes > 0xffffffffull) {
+            C->direct = false;
+            return;
+        }
+        C->direct_host = C->direct_host || host;
+        C->direct_cut = C->direct_cut || cut;
+        for (uint32_t l = 0; l < V.layout.nb_levels; ++l) {
+            StoreLevel &S = C->stores.level[V.level_base + l];
+            S.store = host ? reinterpret_cast<uint64_t>(V.src.dev) + V.src.level_off[l] : 0u;
+            S.nbx = V.layout.nb_bricks[l][0];
+            S.nby = V.layout.nb_bricks[l][1];
+            S.bytes = static_cast<uint32_t>(V.big_bytes);
+            S.cut = cut ? (v << 6 | l) + 1u : 0u;
+        }
+    }
 }
 
 static bool has_source(const gc_cache *C) {

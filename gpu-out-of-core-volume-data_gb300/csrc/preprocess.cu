@@ -687,12 +687,22 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
 // brick source): job j = big brick (x, y, z) of level `lvl` of volume `vol`
 // into staging slot `slot`; one block per job, its warps over the job's small
 // bricks, each by the level bricker's rule.
+// list: the jobs are the elements of a miss list instead, j into slot j (volumes
+// whose big bricks are one brick each; elements of other volumes are skipped).
 __global__ void __launch_bounds__(256) cut_bricks_kernel(const CutSources srcs, const uint4 *__restrict__ jobs,
-                                                         uint32_t n, uint8_t *__restrict__ staging,
-                                                         uint64_t stride) {
+                                                         const uint4 *__restrict__ list, const StoreMap m, uint32_t n,
+                                                         uint8_t *__restrict__ staging, uint64_t stride) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (uint32_t j = blockIdx.x; j < n; j += gridDim.x) {
-        const uint4 job = jobs[j];
+        uint4 job;
+        if (list) {
+            job = list[j];
+            const StoreLevel &l = m.level[job.w];
+            if (l.cut == 0u) continue;
+            job.w = (j << 8) | (l.cut - 1u);
+        } else {
+            job = jobs[j];
+        }
         const uint32_t lvl = job.w & 63u, vol = (job.w >> 6) & 3u, slot = job.w >> 8;
         const CutSource &cs = srcs.vol[vol];
         BrickParams p = cs.p;
@@ -708,10 +718,10 @@ __global__ void __launch_bounds__(256) cut_bricks_kernel(const CutSources srcs, 
     }
 }
 
-void launch_cut_bricks(const CutSources &srcs, const uint4 *jobs, uint32_t n, uint8_t *staging, uint64_t stride,
-                       cudaStream_t s) {
+void launch_cut_bricks(const CutSources &srcs, const uint4 *jobs, const uint4 *list, const StoreMap &m, uint32_t n,
+                       uint8_t *staging, uint64_t stride, cudaStream_t s) {
     if (n == 0) return;
-    cut_bricks_kernel<<<std::min<uint32_t>(n, static_cast<uint32_t>(sm_count()) * 8), 256, 0, s>>>(srcs, jobs, n,
+    cut_bricks_kernel<<<std::min<uint32_t>(n, static_cast<uint32_t>(sm_count()) * 8), 256, 0, s>>>(srcs, jobs, list, m, n,
                                                                                                  staging, stride);
     GC_CUDA(cudaGetLastError());
     count_launch();
