@@ -20,6 +20,8 @@
 // the scan, cap and decode in one pass of its own blocks.
 // Every wait for a predecessor's count is bounded; on expiry the kernel sets
 // ScanCtl::err.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -149,6 +151,56 @@ __global__ void __launch_bounds__(kThreads) lru_partition_kernel(const uint32_t 
         for (uint32_t j = threadIdx.x; j < gridDim.x; j += kThreads) status[j] = 0;
         if (threadIdx.x == 0) ctl->ticket = ctl->done = 0;
     }
+}
+
+// The whole LRU update of a pool of up to kClusterSlots slots in one launch of one
+// thread-block cluster: every block partitions 1024 kItems slots, and the blocks
+// read one another's counts from distributed shared memory between the two
+// halves, so neither a count kernel before nor waits through memory are needed.
+// Bound by latency -- two dependent loads, a cluster barrier, a store -- so the
+// slots are spread over as many of the eight blocks as there are.  Install frame
+// of a 32,768-slot cache from render to installed bricks: 31 -> 21 us.
+template <uint32_t kItems>
+__global__ void __launch_bounds__(1024) lru_cluster_kernel(const uint32_t *__restrict__ order_in,
+                                                           uint32_t *__restrict__ order_out,
+                                                           const uint32_t *__restrict__ usage, uint32_t ts, uint32_t n,
+                                                           uint32_t *__restrict__ count) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    __shared__ uint32_t s_used[32], s_total;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, block = cluster.block_rank();
+    // a warp's 512 consecutive items, 32 at a time
+    const uint32_t base = block * (1024u * kItems) + warp * (32u * kItems) + lane;
+    uint32_t ids[kItems], mine = 0, used = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) ids[k] = base + 32u * k < n ? __ldg(order_in + base + 32u * k) : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k)
+        mine |= (base + 32u * k < n && usage[ids[k]] == ts ? 1u : 0u) << k;
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) used += __popc(__ballot_sync(0xffffffffu, (mine >> k) & 1u));
+    if (lane == 0) s_used[warp] = used;
+    __syncthreads();
+    const uint32_t of_warp = s_used[lane];
+    if (threadIdx.x < 32u) {
+        const uint32_t total = __reduce_add_sync(0xffffffffu, of_warp);
+        if (lane == 0) s_total = total;
+    }
+    cluster.sync();
+    const uint32_t blocks = cluster.num_blocks();
+    const uint32_t of_block = lane < blocks ? *cluster.map_shared_rank(&s_total, lane) : 0u;
+    uint32_t before = __reduce_add_sync(0xffffffffu, (lane < block ? of_block : 0u) + (lane < warp ? of_warp : 0u));
+    const uint32_t total_used = __reduce_add_sync(0xffffffffu, of_block);
+#pragma unroll
+    for (uint32_t k = 0; k < kItems; ++k) {
+        const uint32_t i = base + 32u * k;
+        const uint32_t flags = __ballot_sync(0xffffffffu, (mine >> k) & 1u);
+        const uint32_t used_before = before + __popc(flags & ((1u << lane) - 1u));
+        if (i < n) order_out[(mine >> k) & 1u ? used_before : total_used + i - used_before] = ids[k];
+        before += __popc(flags);
+    }
+    if (block == 0 && threadIdx.x == 0) *count = total_used;
+    cluster.sync();  // no block ends while another reads its count
 }
 
 // coord_1D_to_3D (CacheManagerKernels.cu:32-72) of an entry (the page directory
@@ -794,6 +846,32 @@ void launch_lru_partition(const uint32_t *order_in, uint32_t *order_out, const u
     lru_partition_kernel<<<lru_tiles(nslots), kThreads, 0, s>>>(order_in, order_out, usage, ts, nslots, count, status,
                                                                 ctl);
     GC_CUDA(cudaGetLastError());
+    count_launch();
+}
+
+void launch_lru_cluster(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
+                        uint32_t nslots, uint32_t *count, cudaStream_t s) {
+    static_assert(kClusterSlots == 8u * 16u * 1024u, "a portable cluster has up to 8 blocks");
+    uint32_t items = 1;
+    while (items < 16u && items * 8192u < nslots) items *= 2u;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(div_up(nslots, 1024u * items));
+    cfg.blockDim = dim3(1024);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cfg.gridDim.x;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto go = [&](auto kernel) { GC_CUDA(cudaLaunchKernelEx(&cfg, kernel, order_in, order_out, usage, ts, nslots, count)); };
+    switch (items) {
+        case 1: go(lru_cluster_kernel<1>); break;
+        case 2: go(lru_cluster_kernel<2>); break;
+        case 4: go(lru_cluster_kernel<4>); break;
+        case 8: go(lru_cluster_kernel<8>); break;
+        default: go(lru_cluster_kernel<16>); break;
+    }
     count_launch();
 }
 

@@ -600,10 +600,14 @@ static void lru_update(gc_cache *C, cudaStream_t s, int scan_slot = -1, bool mar
     a.status = C->status_miss;
     a.ctl = C->ctl_miss;
     a.silent_tile = 0xffffffffu;
-    a.usage[0] = C->usage;
-    a.nslots[0] = C->nslots;
-    a.count[0] = C->d_count;
-    if (C->pt.shift) {  // its counter word is pt_njobs, free between installs
+    // pools of one cluster count their used slots themselves
+    const bool small = C->nslots <= kClusterSlots, pt_small = C->pt_slots <= kClusterSlots;
+    if (!small) {
+        a.usage[0] = C->usage;
+        a.nslots[0] = C->nslots;
+        a.count[0] = C->d_count;
+    }
+    if (C->pt.shift && !pt_small) {  // its counter word is pt_njobs, free between installs
         a.usage[1] = C->pt.usage;
         a.nslots[1] = C->pt_slots;
         a.count[1] = C->pt_njobs;
@@ -619,21 +623,28 @@ static void lru_update(gc_cache *C, cudaStream_t s, int scan_slot = -1, bool mar
         a.mx = C->mx;
         a.my = C->my;
     }
-    launch_frame_scan(a, C->lt, s);
+    if (a.nscan || a.nslots[0] || a.nslots[1]) launch_frame_scan(a, C->lt, s);
     if (scan_slot >= 0) {
         gc_cache::MissList &L = C->lists[scan_slot];
         if (mark)
             launch_mark_in_flight(L.d, C->ctl_miss, C->d.max_requests, C->lt, C->mx, C->my, C->nentries, C->mrpd, s);
         GC_CUDA(cudaEventRecord(L.ev, s));
     }
-    launch_lru_partition(C->order[C->cur], C->order[C->cur ^ 1], C->usage, C->ts, C->nslots, C->d_count,
-                         C->status_lru, C->ctl_lru, s);
+    if (small)
+        launch_lru_cluster(C->order[C->cur], C->order[C->cur ^ 1], C->usage, C->ts, C->nslots, C->d_count, s);
+    else
+        launch_lru_partition(C->order[C->cur], C->order[C->cur ^ 1], C->usage, C->ts, C->nslots, C->d_count,
+                             C->status_lru, C->ctl_lru, s);
     C->cur ^= 1;
     if (C->pt.shift) {
         // the table pool's LRU (CacheManager::lru_update's loop over the
         // table caches, CacheManager.hpp:386-406)
-        launch_lru_partition(C->pt_order[C->pt_cur], C->pt_order[C->pt_cur ^ 1], C->pt.usage, C->ts, C->pt_slots,
-                             C->pt_njobs, C->status_pt, C->ctl_pt, s);
+        if (pt_small)
+            launch_lru_cluster(C->pt_order[C->pt_cur], C->pt_order[C->pt_cur ^ 1], C->pt.usage, C->ts, C->pt_slots,
+                               C->pt_njobs, s);
+        else
+            launch_lru_partition(C->pt_order[C->pt_cur], C->pt_order[C->pt_cur ^ 1], C->pt.usage, C->ts, C->pt_slots,
+                                 C->pt_njobs, C->status_pt, C->ctl_pt, s);
         C->pt_cur ^= 1;
     }
 }

@@ -1,5 +1,5 @@
 """The frame's scans -- request scan, used-slot counts and the LRU partition -- at
-the edges of their tiles (8192 request entries, 4096 slots): one entry or slot
+the edges of their tiles (8192 request entries, 1024 to 16,384 slots): one entry or slot
 more or less than a whole number of tiles, flags at the first and last entries of
 a tile, none, all, and more than the list holds.  Lists, totals and LRU order
 equal a numpy restatement."""
@@ -41,9 +41,14 @@ def test_miss_list_at_tile_edges(gc, torch_cuda, n, maxreq):
         assert (got[k:] == -1).all()
 
 
-@pytest.mark.parametrize("slots", [(1, 1, 1), (31, 1, 1), (4095, 1, 1), (16, 16, 16), (4097, 1, 1), (64, 64, 3)])
+# one cluster of up to eight blocks (1024, 2048, ... 16,384 slots each, 131,072 in all) and
+# the count + partition kernels above
+@pytest.mark.parametrize("slots", [(1, 1, 1), (31, 1, 1), (4095, 1, 1), (16, 16, 16), (4097, 1, 1), (64, 64, 3), (1024, 1, 1), (1025, 1, 1), (64, 64, 2), (8193, 1, 1), (16385, 1, 1),
+                                   (128, 128, 1), (128, 64, 5), (128, 128, 8), (131073, 1, 1),
+                                   (64, 64, 64), (262145, 1, 1), (270000, 1, 1)])
 def test_lru_order_at_tile_edges(gc, torch_cuda, slots):
-    vol = gc.volume_desc((64, 64, 64), 16, 1, 1)
+    B = 16 if slots[0] * slots[1] * slots[2] < 20000 else 4
+    vol = gc.volume_desc((64, 64, 64), B, 1, 1)
     layout = gc.compute_layout(vol)
     cm = gc.CacheManager(vol, layout, slots, max_requests=1)
     cm.set_source_callback(lambda *a: gc.BRICK_UNKNOWN)
@@ -62,7 +67,7 @@ def test_lru_order_at_tile_edges(gc, torch_cuda, slots):
         lru = np.zeros(n, dtype=np.dtype([("c", np.uint32, 3), ("level", np.uint32), ("v", np.float32, 3)]))
         cm.dump(gc.DUMP_LRU, lru)
         sx, sy = slots[0], slots[1]
-        want = np.stack([(order % sx) * 16, (order // sx % sy) * 16, (order // (sx * sy)) * 16], 1)
+        want = np.stack([(order % sx) * B, (order // sx % sy) * B, (order // (sx * sy)) * B], 1)
         assert np.array_equal(lru["c"], want), share
         assert cm.stats().last_used == used.sum()
     assert cm.stats().device_error == 0
