@@ -1029,9 +1029,9 @@ __device__ __forceinline__ void retire_warp(uint32_t *queue, uint32_t nwarps) {
 // few rays.  Refilling a warp's idle lanes once 1 / 8 / 16 / all 32 are idle:
 // 6.5 / 5.1 / 4.6 / 3.8 ms for the first of these frames.
 // N: samples a ray takes at a time (ray_sample).  N = 2 at 80 registers (24
-// resident warps per SM) for launches of many rays, bound by issue; N = 4 with
-// all the registers it needs for launches of few rays, bound by latency
-// (render_launch_config).
+// resident warps per SM) for launches of many rays, bound by issue; N = 6 (two
+// channels 4) with all the registers it needs for launches of few rays, bound by
+// latency (render_launch_config).
 // ONE: a launch of one view, whose parameters come with the launch (`one`: no
 // table upload, read from constant memory) and whose visible bins each block
 // works out for itself (no kernel before this one).  The first tile of a warp is
@@ -1106,7 +1106,8 @@ void *march_kernel_bs(uint32_t kind) {
         case 2: return reinterpret_cast<void *>(render_kernel<uint16_t, BS, TL, N, ONE>);
         case 4: return reinterpret_cast<void *>(render_kernel<float, BS, TL, N, ONE>);
         case 0: return reinterpret_cast<void *>(render_kernel<MixedVoxel, BS, TL, N, ONE>);
-        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N, ONE>);
+        // (two channels hold twice the values a sample)
+        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N < 4 ? N : 4, ONE>);
         default: return nullptr;
     }
 }
@@ -1120,7 +1121,7 @@ void *march_kernel_n(uint32_t kind, uint32_t brick_size, bool two_level) {
 }
 void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShape shape) {
     switch (shape) {
-        case MarchShape::kOneFew: return march_kernel_n<4, true>(kind, brick_size, two_level);
+        case MarchShape::kOneFew: return march_kernel_n<6, true>(kind, brick_size, two_level);
         case MarchShape::kOneMany: return march_kernel_n<2, true>(kind, brick_size, two_level);
         default: return march_kernel_n<2, false>(kind, brick_size, two_level);
     }
@@ -1212,7 +1213,7 @@ constexpr uint32_t kTwoChannelU8 = 0x202;
 static uint32_t voxel_kind(const CacheView &cv) { return cv.nc == 2 ? kTwoChannelU8 : cv.eb; }
 
 static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool two_level, uint32_t total_tiles,
-                                         uint32_t rect_tiles, bool one) {
+                                         uint32_t rect_tiles, bool one, bool long_rays) {
     const RenderTuning tune = render_tuning();
     const uint32_t threads = tune.threads;
     GC_REQUIRE(threads == 64 || threads == 128 || threads == 256, "render threads must be 64, 128 or 256");
@@ -1220,14 +1221,18 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
     // widths share the cache; two 8-bit channels with a 2D transfer function)
     // from the exact or the fast build
     const bool fast_build = tune.precision == 1;
-    // Few rays: the tiles that can hold rays meeting the box fit in one wave of
-    // the resident warps, so the launch lasts as long as its longest tile and a
-    // ray's own latency counts, not the number of resident warps.  Measured (4
-    // samples at a time / 2): 464 such tiles 121 / 136 us, 1,950 tiles 336 / 408 us
-    // a frame; 13,622 tiles 2.21 / 2.14 ms, 30,592 tiles 2.90 / 2.73 ms, 63,120
-    // tiles 6.27 / 5.32 ms.
+    // Few rays: the launch lasts about as long as its longest tiles, and a ray's
+    // own latency counts, not the number of resident warps.  A launch at N = 2 / 4 /
+    // 6 samples at a time, by its tiles that can hold rays meeting the box: DVR
+    // 256^3 u8 700 tiles 198 / 152 / 138 us, 1,950 334 / 255 / 232, 4,700 365 / 305 /
+    // 293; DVR 512^3 u16 2,600 579 / 457 / 408, 4,650 862 / 653 / 719, 7,300 963 /
+    // 863 / 1004; maximum intensity 2,600 496 / 410 / 390, 4,650 514 / 591 / 563; two
+    // channels 1,200 519 / 436, 2,600 661 / 659, 4,650 913 / 936.  So N = 6 (two
+    // channels 4) up to one wave of the N = 2 kernel's 24 warps per SM, DVR of one
+    // channel up to one and a half.
     // Launches of several views take the shape for many rays.
-    const bool few = one && rect_tiles <= static_cast<uint32_t>(sm_count()) * kWideWarps;
+    const uint32_t few_warps = long_rays ? kWideWarps * 3u / 2u : kWideWarps;
+    const bool few = one && rect_tiles <= static_cast<uint32_t>(sm_count()) * few_warps;
     const MarchShape shape = few ? MarchShape::kOneFew : (one ? MarchShape::kOneMany : MarchShape::kSeveral);
     void *kernel = fast_build ? fast::march_kernel(eb, brick_size, two_level, shape)
                               : exact::march_kernel(eb, brick_size, two_level, shape);
@@ -1252,7 +1257,7 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
 void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev, uint32_t nviews,
                    uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
     ViewParams none{};
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &none, &views_dev, &nviews,
@@ -1264,7 +1269,8 @@ void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams 
 void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewParams &view, uint32_t total_tiles,
                        uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, true);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, true,
+                                                view.mode == GC_MODE_DVR && cv.nc == 1);
     uint32_t nwarps = L.grid * (L.threads / 32), nviews = 1;
     const ViewParams *views = nullptr;
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), const_cast<ViewParams *>(&view),
@@ -1294,7 +1300,7 @@ void launch_render_graph(RenderGraph &g, const CacheView &cv, const LevelTables 
                          const ViewParams *views_pinned, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
                          uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
     const ViewParams *vd = views_dev;
     ViewParams none{};

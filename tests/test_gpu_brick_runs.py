@@ -189,6 +189,24 @@ def test_launches_of_few_and_many_rays_agree(gc, torch_cuda, kind, mode, sampler
     for x, y, z in zip(one, many, mixed):
         assert np.array_equal(x, y) and np.array_equal(x, z)
 
+    # one view of many rays, alone and beside another view
+    W, H = 640, 400
+    assert W * H // 32 > 36 * t.cuda.get_device_properties(0).multi_processor_count
+    bufs = [(t.zeros(W * H, dtype=t.int32, device="cuda"), t.zeros(W * H, device="cuda"),
+             t.zeros(W * H * 4, device="cuda"))]
+    large = gc.make_view(scenario.orbit_camera(gc, 3, 12, 1.4), W, H, tf_dev.data_ptr(), tf.shape[-2],
+                         bufs[0][0].data_ptr(), bufs[0][1].data_ptr(), bufs[0][2].data_ptr(), focal=0.9,
+                         early_alpha=0.99, mode=mode, sampler=sampler, tf_height=tf.shape[0] if ch == 2 else 0)
+    for _ in range(100):
+        cm.render(large)
+        if cm.update():
+            break
+    alone = images(lambda: cm.render(large))
+    beside = images(lambda: cm.render_batch([large, views[0]]))
+    assert alone[0].any()
+    for x, y in zip(alone, beside):
+        assert np.array_equal(x, y)
+
 
 @pytest.mark.parametrize("width", [1, 2, 256, 512, 513])
 def test_visible_bins_of_either_launch_agree(gc, torch_cuda, width):
