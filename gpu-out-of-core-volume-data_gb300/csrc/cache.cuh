@@ -101,7 +101,7 @@ struct CacheView {
 // entry, and a view the bins its transfer function can make visible.  A brick
 // whose bins are all invisible contributes no sample above the compositing
 // threshold, so the march steps through it without sampling (same t
-// sequence, same image).
+// sequence, same image).  Bricks of two 8-bit channels record 32 bins of each.
 constexpr uint32_t kValueBins = 64;
 
 // Per-launch ray-caster parameters of one view.
@@ -136,6 +136,7 @@ struct ViewParams {
     uint32_t nlevels;                   // levels of the view's volume
     uint32_t eb;                        // bytes per voxel of the view's volume
     uint32_t fallback;                  // sample a coarser mapped level where a brick is missing (preview)
+    uint32_t skip_two;                  // step through invisible bricks (DVR, two 8-bit channels)
     uint32_t skip_max;                  // maximum intensity, one channel: step through bricks that cannot
                                         // raise the maximum
     float cell_margin, run_margin;      // margins of the ray caster's run through one brick (run_bound)

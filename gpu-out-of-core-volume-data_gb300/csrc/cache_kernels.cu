@@ -440,6 +440,33 @@ __device__ unsigned long long block_bins_from(float lo, float hi) {
     }
     return bins_of_range(lo, hi);
 }
+// Two 8-bit channels: 32 bins each, channel 0 in the low half.  mn and mx hold the
+// thread's bounds, channel 0 in the low 16 bits; the result is valid in thread 0.
+__device__ unsigned long long block_bins_of_two(uint32_t mn, uint32_t mx) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mn = min_u16x2(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+        mx = max_u16x2(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    }
+    __shared__ uint32_t s_mn[9], s_mx[9];
+    const uint32_t warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31u) == 0) {
+        s_mn[warp] = mn;
+        s_mx[warp] = mx;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return 0;
+    for (uint32_t w = 1; w < (blockDim.x + 31) / 32; ++w) {
+        mn = min_u16x2(mn, s_mn[w]);
+        mx = max_u16x2(mx, s_mx[w]);
+    }
+    auto bins = [](uint32_t lo, uint32_t hi) {  // bin of v: floor(32 v / 255), at most 31; one more on either side
+        const uint32_t b0 = min(lo * 32u / 255u, 31u), b1 = min(min(hi * 32u / 255u, 31u) + 1u, 31u);
+        const uint32_t upto = b1 == 31u ? ~0u : (2u << b1) - 1u;
+        return upto & ~((1u << (b0 ? b0 - 1u : 0u)) - 1u);
+    };
+    return bins(mn & 0xffffu, mx & 0xffffu) | static_cast<unsigned long long>(bins(mn >> 16, mx >> 16)) << 32;
+}
 template <class At>
 __device__ unsigned long long block_value_bins(uint32_t nvox, uint32_t eb, At at) {
     float lo = 3.4e38f, hi = -3.4e38f;
@@ -638,8 +665,9 @@ __global__ void __launch_bounds__(kCopyThreads + 32) install_place_kernel(Instal
         // (one read of the brick for both)
         const uint32_t qs = __ffs(vec_per_row) - 1u, bs = __ffs(B) - 1u;
         const uint32_t nvec = rows * vec_per_row;
-        const bool bins = a.slot_bins && a.nc == 1;
+        const bool bins = a.slot_bins && a.nc == 1, two = a.slot_bins && a.nc == 2 && eb == 2;
         float lo = 3.4e38f, hi = -3.4e38f;
+        ValueRange<1> range;  // two 8-bit channels: even and odd bytes
         for (uint32_t v0 = tid < kCopyThreads ? tid : nvec; v0 < nvec; v0 += 4u * kCopyThreads) {
             uint4 val[4];
 #pragma unroll
@@ -659,12 +687,18 @@ __global__ void __launch_bounds__(kCopyThreads + 32) install_place_kernel(Instal
                 if (v < nvec) {
                     reinterpret_cast<uint4 *>(dst)[v] = val[u];
                     if (bins) chunk_range(val[u], eb, lo, hi);
+                    if (two) range.add(val[u]);
                 }
             }
         }
         if (!a.slot_bins) return;
+        if (two) {
+            const unsigned long long b2 = block_bins_of_two(range.mn_channels(), range.mx_channels());
+            if (threadIdx.x == 0) a.slot_bins[slot] = b2;
+            return;
+        }
         if (a.nc != 1) {
-            if (threadIdx.x == 0) a.slot_bins[slot] = ~0ull;  // several channels: never skipped
+            if (threadIdx.x == 0) a.slot_bins[slot] = ~0ull;  // never skipped
             return;
         }
         const unsigned long long b2 = block_bins_from(lo, hi);
@@ -682,7 +716,7 @@ __global__ void __launch_bounds__(kCopyThreads + 32) install_place_kernel(Instal
     if (!a.slot_bins) return;
     __syncthreads();
     if (a.nc != 1) {
-        if (threadIdx.x == 0) a.slot_bins[slot] = ~0ull;  // several channels: never skipped
+        if (threadIdx.x == 0) a.slot_bins[slot] = ~0ull;  // never skipped
         return;
     }
     const unsigned long long bins = block_value_bins(B * B * B, eb, [&](uint32_t v) { return dst + v * eb; });

@@ -38,6 +38,7 @@
 #include "brickfiles.h"
 #include "cache.cuh"
 #include "gc_internal.h"
+#include "view_bins.cuh"
 
 namespace gc {
 
@@ -806,6 +807,8 @@ static void fill_view(const gc_cache *C, const gc_view &in, ViewParams &out) {
     out.tfh = in.tf_height > 0 ? in.tf_height : 1;
     // empty-space skipping: DVR of one channel through a 1D transfer function
     out.skip_empty = in.mode == GC_MODE_DVR && V.desc.channels == 1 ? render_tuning().skip_empty : 0u;
+    // or of two 8-bit channels through a 2D one (launches of one view)
+    out.skip_two = in.mode == GC_MODE_DVR && V.desc.channels == 2 && in.tf_height <= kTwoBinRows ? render_tuning().skip_empty : 0u;
     // and maximum intensity of one channel of integer voxels
     out.skip_max = in.mode == GC_MODE_MOP && V.desc.channels == 1 && V.desc.encoded_bytes <= 2
                        ? render_tuning().skip_empty

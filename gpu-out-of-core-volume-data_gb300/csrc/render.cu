@@ -326,6 +326,15 @@ __device__ __forceinline__ bool brick_below(unsigned long long bins, float max_o
     return top < 63 && static_cast<float>(top + 1) * (1.0f / kValueBins) <= max_op;
 }
 
+// Two 8-bit channels: true when a brick with these value bins (the install's: 32
+// of channel 0, then 32 of channel 1) shows nothing; rows[b]: the bins of channel
+// 1 visible with bin b of channel 0.
+__device__ __forceinline__ bool two_invisible(unsigned long long bins, const uint32_t *rows) {
+    uint32_t seen = 0;
+    for (uint32_t b = static_cast<uint32_t>(bins); b; b &= b - 1u) seen |= rows[__ffs(static_cast<int>(b)) - 1];
+    return (seen & static_cast<uint32_t>(bins >> 32)) == 0u;
+}
+
 enum Status { kMapped = 0, kUnmapped = 1, kEmpty = 2, kInvisible = 3, kCoarser = 4 };
 
 // Per-thread page-walk state (K_CacheManager::_previousCoords / _previousEntries).
@@ -484,10 +493,13 @@ __device__ __forceinline__ uint4 load_entry(const CacheView &cv, const LevelTabl
 // kMapped leaves the brick to sample in w.base and its level in slvl.
 // max_op: the maximum so far of a maximum-intensity ray that skips bricks
 // (brick_below), else -1.
+// two_rows: the view's visible bins of two channels, or null (one channel, or
+// nothing is skipped).
 template <bool TL>
 __device__ __forceinline__ int visit(const CacheView &cv, const LevelTables &lt, const ViewParams &vp, uint32_t lvl,
                                      uint32_t lvl_end, V3 np, uint32_t idx, uint3 q, float max_op,
-                                     unsigned long long visible, Walk &w, uint32_t &slvl) {
+                                     unsigned long long visible, const uint32_t *two_rows, Walk &w,
+                                     uint32_t &slvl) {
     // read where used (rare path): the view's fallback flag (a missing brick)
     if (idx != w.pidx) {
         // A new entry: the entry and its value bins are read together (one
@@ -500,6 +512,7 @@ __device__ __forceinline__ int visit(const CacheView &cv, const LevelTables &lt,
         w.invisible = (bins & visible) == 0ull && (e.w == 1u || (e.w == 0u && cv.bins_user));
         if (e.w == 1u) {
             if (max_op >= 0.f) w.invisible = w.invisible || brick_below(bins, max_op);
+            if (two_rows) w.invisible = two_invisible(bins, two_rows);
             const uint32_t B = cv.B;
             const uint32_t slot = cv.b_shift < 32u ? (e.x >> cv.b_shift) + (e.y >> cv.b_shift) * cv.sx +
                                                          (e.z >> cv.b_shift) * cv.sx * cv.sy
@@ -748,9 +761,9 @@ __device__ __forceinline__ float run_bound(const LevelTables &lt, const Ray &r, 
 // or it stepped through an invisible or empty brick.
 // ONE: the view's visible bins are kept in shared memory (`visible`), else in
 // its parameters.
-template <bool TL, bool ONE>
+template <bool TL, bool ONE, bool TWO>
 __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables &lt, const unsigned long long *visible,
-                                         Ray &r) {
+                                         const uint32_t *two_rows, Ray &r) {
     const ViewParams &vp = *r.vp;
     if (!((!r.dvr || r.fc.w < r.early) && r.t < r.tfar)) return false;
     const V3 np = norm_pos(r.pos);
@@ -782,7 +795,7 @@ __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables 
     uint3 q;
     const uint32_t idx = entry_index(cv, lt, r.lvl, np, p, q);
     const int st = visit<TL>(cv, lt, vp, r.lvl, r.lvl_end, np, idx, q, vp.skip_max ? r.maxOp : -1.0f,
-                             ONE ? *visible : vp.visible, r.w, r.slvl);
+                             TWO ? ~0ull : (ONE ? *visible : vp.visible), ONE && TWO ? two_rows : nullptr, r.w, r.slvl);
     if (st == kUnmapped) {
         vp.tbuf[r.i] = r.t;
         if (r.dvr)
@@ -922,10 +935,11 @@ __device__ __forceinline__ void ray_sample(const CacheView &cv, const LevelTable
 // ray ended.
 template <typename T, uint32_t BS, bool TL, int N, bool ONE>
 __device__ __forceinline__ bool ray_round(const CacheView &cv, const LevelTables &lt,
-                                          const unsigned long long *visible, const float4 *pairs, Ray &r,
+                                          const unsigned long long *visible, const uint32_t *two_rows,
+                                          const float4 *pairs, Ray &r,
                                           bool active) {
     bool ended = false;
-    if (active && !r.pend) ended = !ray_walk<TL, ONE>(cv, lt, visible, r);
+    if (active && !r.pend) ended = !ray_walk<TL, ONE, std::is_same<T, TwoU8>::value>(cv, lt, visible, two_rows, r);
     __syncwarp();
     if (active && r.pend) ray_sample<T, BS, N, ONE>(cv, lt, pairs, r);
     __syncwarp();
@@ -1046,9 +1060,14 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
     __shared__ unsigned long long s_visible, s_samples[8], s_rays[8];  // of each warp
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (lane == 0) s_samples[warp] = s_rays[warp] = 0;
-    extern __shared__ float4 s_pairs[];  // ONE, one channel: 2 (tfw + 4)
-    if constexpr (ONE) {
-        if constexpr (!std::is_same<T, TwoU8>::value) fill_pairs(one.tf, one.tfw, s_pairs);
+    extern __shared__ float4 s_pairs[];  // ONE: 2 (tfw + 4), or 8 tfh with two channels (scratch)
+    constexpr bool TWO = std::is_same<T, TwoU8>::value;
+    __shared__ uint32_t s_two[TWO ? 32 : 1];
+    if constexpr (ONE && TWO) {
+        visible_bins_of_two(one, s_two, reinterpret_cast<float *>(s_pairs));
+        __syncthreads();
+    } else if constexpr (ONE) {
+        fill_pairs(one.tf, one.tfw, s_pairs);
         if (threadIdx.x < 32u) {
             const unsigned long long v = visible_bins(one, lane);
             if (lane == 0) s_visible = v;
@@ -1068,7 +1087,7 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
         bool active = x < vp->W && y < vp->H && ray_setup<T>(lt, vp, x, y, r);
         if (active) marched = ray_enters(r);
         while (__any_sync(0xffffffffu, active)) {
-            if (ray_round<T, BS, TL, N, ONE>(cv, lt, &s_visible, s_pairs, r, active)) {
+            if (ray_round<T, BS, TL, N, ONE>(cv, lt, &s_visible, s_two, s_pairs, r, active)) {
                 active = false;
                 unm = ray_finish(r);
                 coarse_any = r.coarse;
@@ -1275,7 +1294,7 @@ void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewPar
     const ViewParams *views = nullptr;
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), const_cast<ViewParams *>(&view),
                     &views, &nviews, &total_tiles, &queue, &nwarps};
-    const size_t pairs = cv.nc == 1 ? (view.tfw + 4u) * 2u * sizeof(float4) : 0u;
+    const size_t pairs = cv.nc == 1 ? (view.tfw + 4u) * 2u * sizeof(float4) : (view.skip_two ? view.tfh * 32u * sizeof(float) : 0u);
     GC_CUDA(cudaLaunchKernel(L.func, dim3(L.grid), dim3(L.threads), args, pairs, s));
     count_launch();
 }

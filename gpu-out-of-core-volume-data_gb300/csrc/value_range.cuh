@@ -49,6 +49,14 @@ struct ValueRange {
         const uint32_t m = EB == 1 ? max_u16x2(mx0, mx1) : mx0;
         return max(m & 0xffffu, m >> 16);
     }
+    // EB 1, two interleaved 8-bit channels (even and odd bytes): the bounds of
+    // channel 0 in the low 16 bits, of channel 1 in the high ones
+    __device__ __forceinline__ uint32_t mn_channels() const {
+        return min(mn0 & 0xffffu, mn0 >> 16) | min(mn1 & 0xffffu, mn1 >> 16) << 16;
+    }
+    __device__ __forceinline__ uint32_t mx_channels() const {
+        return max(mx0 & 0xffffu, mx0 >> 16) | max(mx1 & 0xffffu, mx1 >> 16) << 16;
+    }
     // as the ray caster's samplers normalize them (monotone, so the range of the
     // normalized values)
     __device__ __forceinline__ void normalized(float &lo, float &hi) const {

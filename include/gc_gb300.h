@@ -543,9 +543,10 @@ int gc_render_precision_get(int *precision);
  * DVR view of a one-channel volume the value range its transfer function can
  * make visible; a ray steps through a brick with no visible value without
  * sampling it (the same t steps; samples there stay below the 0.001
- * compositing threshold).  A maximum-intensity ray of a one-channel volume of
- * integer voxels steps likewise through a brick whose range cannot raise its
- * maximum.  No counterpart in the reference. */
+ * compositing threshold).  Launches of one view step likewise through bricks of
+ * two 8-bit channels that a 2D transfer function of up to 64 rows cannot make
+ * visible.  A maximum-intensity ray of a one-channel volume of
+ * integer voxels steps through a brick whose range cannot raise its maximum.  No counterpart in the reference. */
 int gc_render_empty_skip(int enable);
 
 /* ------------------------------------------------------------------------ */

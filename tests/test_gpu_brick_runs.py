@@ -249,3 +249,59 @@ def test_visible_bins_of_either_launch_agree(gc, torch_cuda, width):
     for x, y in zip(*got):
         assert np.array_equal(x, y)
     assert got[0][3] > 0
+
+
+@pytest.mark.parametrize("B,width,height,fewer", [(16, 64, 48, True), (8, 64, 64, True), (8, 33, 1, True), (16, 5, 7, True),
+                                                  (16, 64, 65, False), (16, 600, 8, False), (4, 64, 48, False)])
+@pytest.mark.parametrize("sampler", [0, 1])
+def test_two_channel_skips_change_nothing(gc, torch_cuda, B, width, height, fewer, sampler):
+    """Bricks of two 8-bit channels that the 2D transfer function cannot make
+    visible are stepped through: image, t and state equal those without skipping,
+    bit for bit; nothing is skipped with more than 64 table rows, tables too wide
+    for shared memory, or brick rows of no whole 16 bytes."""
+    t = torch_cuda
+    n = 48
+    z, y, x = np.meshgrid(*[np.linspace(-1, 1, n)] * 3, indexing="ij")
+    rng = np.random.default_rng(2)
+    c0 = np.clip(255 * np.exp(-3 * (x * x + y * y + z * z)) + rng.uniform(0, 8, (n, n, n)), 0, 255)
+    c1 = np.clip(127 + 127 * np.sin(3 * x + 2 * y) + rng.uniform(-9, 9, (n, n, n)), 0, 255)
+    d = t.from_numpy(np.stack([c0, c1], -1).astype(np.uint8).reshape(-1)).cuda()
+    vol = gc.volume_desc((n, n, n), B, 1, 2, 2)
+    layout = gc.compute_layout(vol)
+    while tuple(layout.mip[layout.nb_levels - 1]) != tuple(layout.initial[layout.nb_levels - 1]):
+        layout.nb_levels -= 1
+    store, offs, _ = gc.pre_process(vol, layout, d)
+    u, v = np.linspace(0, 1, width)[None, :], np.linspace(0, 1, height)[:, None]
+    tf = np.zeros((height, width, 4), np.float32)
+    tf[..., :3] = 0.5
+    tf[..., 3] = np.where((u > 0.45) & (u < 0.8), 0.4, 0.0) * (1.0 if height < 4 else np.where(v > 0.4, 1.0, 0.0))
+    tf_dev = t.from_numpy(tf.reshape(-1)).cuda()
+    images, samples = [], []
+    for skip in (False, True):
+        cm = gc.CacheManager(vol, layout, (32, 32, 32), max_requests=4000)
+        cm.set_source_host(store, offs)
+        W, H = 57, 43
+        b = (t.zeros(W * H, dtype=t.int32, device="cuda"), t.zeros(W * H, device="cuda"),
+             t.zeros(W * H * 4, device="cuda"))
+        view = gc.make_view(scenario.orbit_camera(gc, 1, 12, 2.4), W, H, tf_dev.data_ptr(), width, b[0].data_ptr(),
+                            b[1].data_ptr(), b[2].data_ptr(), sampler=sampler, tf_height=height)
+        gc.render_empty_skip(skip)
+        try:
+            for _ in range(200):
+                cm.render(view)
+                if cm.update():
+                    break
+            for a in b[1:]:
+                a.zero_()
+            before = cm.stats().samples
+            cm.render(view)
+            t.cuda.synchronize()
+            samples.append(cm.stats().samples - before)
+        finally:
+            gc.render_empty_skip(True)
+        images.append([a.cpu().numpy() for a in b])
+        cm.close()
+    for p, q in zip(*images):
+        assert np.array_equal(p, q)
+    assert images[0][0].any()
+    assert samples[1] < samples[0] if fewer else samples[1] == samples[0]
