@@ -315,7 +315,7 @@ struct RenderTuning {
 };
 RenderTuning &render_tuning();
 // What a ray-caster launch holds: one view with few or many rays, or several views.
-enum class MarchShape { kOneFew, kOneMany, kSeveral };
+enum class MarchShape { kOneFew, kOneMany, kOneManyTrilinear, kSeveral };
 // Ray-caster kernels of a voxel kind (1, 2, 4 bytes; 0 mixed widths; 0x202
 // two 8-bit channels) and brick size (16 and 32 have kernels
 // compiled for them; a two-level page directory has kernels of its own),

@@ -238,19 +238,12 @@ struct VoxelTraits<float> {
 // With covering >= 1 both voxels lie in the brick; with covering 0 the lower
 // one is clamped to the brick edge (the reference then reads the neighbouring
 // slot of its texture).
-// BS: the brick size when known at compile time (its row and slice strides
-// become immediate load offsets; bricks with a covering only, so that no voxel is
-// clamped), 0 for the run-time B.
+// i0: the voxel e - 1 in the brick.  BS: the brick size when known at compile
+// time (its row and slice strides become immediate load offsets), 0 for the
+// run-time B.
 template <typename T, uint32_t BS>
-__device__ __forceinline__ float sample_corner(const T *__restrict__ b, uint32_t Brt, uint32_t lx, uint32_t ly,
-                                               uint32_t lz) {
+__device__ __forceinline__ float sample_corner(const T *__restrict__ b, uint32_t Brt, uint32_t i0) {
     const uint32_t B = BS ? BS : Brt;
-    if constexpr (BS == 0) {
-        lx = lx > 0 ? lx : 1u;
-        ly = ly > 0 ? ly : 1u;
-        lz = lz > 0 ? lz : 1u;
-    }
-    const uint32_t i0 = ((lz - 1) * B + (ly - 1)) * B + (lx - 1);
     // the four x pairs of the 2x2x2 block: rows y, y+1 of slices z, z+1
     const T *p0 = b + i0;
     const T *p1 = p0 + B, *p2 = p0 + B * B;
@@ -266,9 +259,9 @@ __device__ __forceinline__ float sample_corner(const T *__restrict__ b, uint32_t
     }
 }
 
-// x mod (B - 2c) by a multiply-high: with m = ceil(2^32 / d), the high word of
-// x m is floor(x / d) for every x < 2^25 and 2 <= d <= 128 (voxel coordinates
-// are below 2^23, checked at cache creation; m = 0 falls back to %).
+// x div and mod (B - 2c) by a multiply-high: with m = ceil(2^32 / d), the high
+// word of x m is floor(x / d) for every x < 2^25 and 2 <= d <= 128 (voxel
+// coordinates are below 2^23, checked at cache creation; m = 0 falls back to %).
 // BS: the compiled brick size, whose B - 2c always has its m.
 template <uint32_t BS>
 __device__ __forceinline__ uint32_t mod_beff(uint32_t x, uint32_t d, uint32_t m) {
@@ -276,8 +269,35 @@ __device__ __forceinline__ uint32_t mod_beff(uint32_t x, uint32_t d, uint32_t m)
     return x - __umulhi(x, m) * d;
 }
 
-// Trilinear sampler at the fractional position f (voxels of the level); the
-// pair (i0, i0 + 1) is clamped to the brick (only reachable with covering 0).
+// Voxel indices without remainders (kTakesOffset; kernels compiled for a brick
+// size, whose bricks have a covering, so that no voxel is clamped): a voxel
+// coordinate m of the level is left as the bits kFloorBits + m that its floor comes
+// in, and the brick's place in the level, this constant and the covering are one
+// offset, worked out when the ray finds the brick (origin_offset).
+constexpr uint32_t kFloorBits = 0x4B000000u;  // of 2^23
+__device__ __forceinline__ float floor_bits(float v) { return __fadd_rd(v, 8388608.0f); }
+template <uint32_t BS>
+__device__ __forceinline__ uint32_t origin_offset(const CacheView &cv, uint32_t qx, uint32_t qy, uint32_t qz) {
+    constexpr uint32_t all = BS * BS + BS + 1u;
+    return (cv.c - kFloorBits) * all - cv.Beff * ((qz * BS + qy) * BS + qx);
+}
+// The index in the brick; samples past the brick (taken, not used) stay in its
+// last 2 x 2 x 2 voxels.
+template <uint32_t BS>
+__device__ __forceinline__ uint32_t index_of(uint32_t x, uint32_t y, uint32_t z, uint32_t offset) {
+    return min((z * BS + y) * BS + x + offset, BS * BS * BS - (BS * BS + BS + 2u));
+}
+// One axis of the trilinear sampler at the fractional position f (voxels of
+// the level): the lower voxel's bits and the weight of the upper one.
+__device__ __forceinline__ uint32_t tri_bits(float f, float &w) {
+    const float b = floor_bits(f);
+    const float fr = f - (b - 8388608.0f);
+    const bool up = fr >= 0.5f;
+    w = up ? fr - 0.5f : fr + 0.5f;
+    return __float_as_uint(b) - (up ? 0u : 1u);
+}
+// The same with the remainder: the pair (i0, i0 + 1) is clamped to the brick
+// (only reachable with covering 0, which the compiled sizes do not take).
 template <uint32_t BS>
 __device__ __forceinline__ void tri_axis(float f, uint32_t c, uint32_t beff, uint32_t magic, uint32_t B,
                                          uint32_t &i0, float &w) {
@@ -301,10 +321,10 @@ __device__ __forceinline__ float ldv(const T *__restrict__ b, uint32_t i) {
     return static_cast<float>(__ldg(b + i));
 }
 template <typename T, uint32_t BS>
-__device__ __forceinline__ float sample_trilinear(const T *__restrict__ b, uint32_t Brt, uint32_t x0, uint32_t y0,
-                                                  uint32_t z0, float wx, float wy, float wz) {
+__device__ __forceinline__ float sample_trilinear(const T *__restrict__ b, uint32_t Brt, uint32_t i, float wx,
+                                                  float wy, float wz) {
     const uint32_t B = BS ? BS : Brt;
-    const uint32_t i = (z0 * B + y0) * B + x0, BB = B * B;
+    const uint32_t BB = B * B;
     const float c00 = fmad(ldv(b, i + 1) - ldv(b, i), wx, ldv(b, i));
     const float c10 = fmad(ldv(b, i + B + 1) - ldv(b, i + B), wx, ldv(b, i + B));
     const float c01 = fmad(ldv(b, i + BB + 1) - ldv(b, i + BB), wx, ldv(b, i + BB));
@@ -354,6 +374,26 @@ struct Walk {
 // float2 for the 2D transfer function.
 struct MixedVoxel {};
 struct TwoU8 {};
+
+// What a kernel marches: several views (the parameters in device memory), or one
+// view, of either sampler or of the one compiled in (launches of many rays, bound by
+// issue: with both samplers in the kernel -> with one, 1024^2 of a 512^3 u16 volume
+// 2.43 -> 2.37 ms, its paged loop 26.1 -> 24.8 ms, trilinear maximum intensity 3.83 ->
+// 3.72 ms).
+enum class Views { kSeveral, kOne, kOneCorner, kOneTrilinear };
+
+// Which samples take their voxel's place in the brick from one offset per brick
+// (origin_offset) instead of a remainder by B - 2c an axis: they save the
+// remainders, the page walk takes over their work, and the offset is a register
+// more.  Per frame, remainders -> offset, launches of one view: 1920x1080 maximum
+// intensity, trilinear, of a 512x448x288 u8 volume 4.47 -> 3.65 ms; corner sampler,
+// 777x555 with two channels 1.47 -> 1.38 ms, 512^2 with few rays (N = 6) 260 -> 254
+// us, but 1024^2 of a 512^3 u16 volume (N = 2) 2.39 -> 2.42 ms and its paged loop
+// 25.2 -> 26.1 ms: so all but the last, whose samples have least to save.  24 views
+// at a time, corner sampler, B = 32: 22.6 -> 23.0 ms (the views' parameters take every
+// register), so launches of several views keep the remainders too.
+template <typename T, uint32_t BS, bool TRI, int N, bool ONE>
+constexpr bool kTakesOffset = BS != 0 && ONE && (TRI || N > 2 || std::is_same<T, TwoU8>::value);
 template <typename T>
 struct SampleOf {
     using type = float;
@@ -377,27 +417,43 @@ __device__ __forceinline__ float4 classify(const float *tf, const float4 *, uint
 }
 
 // One sample at the level position f (voxels) of the brick at `base`, with the
-// reference's corner sampler or the trilinear one (TRI).
-template <typename T, uint32_t BS, bool TRI>
+// reference's corner sampler or the trilinear one (TRI).  offset: origin_offset
+// of the brick (OFS).
+template <typename T, uint32_t BS, bool TRI, bool OFS>
 __device__ __forceinline__ typename SampleOf<T>::type sample_brick(const uint8_t *__restrict__ base,
-                                                                   const CacheView &cv, V3 f) {
+                                                                   const CacheView &cv, V3 f, uint32_t offset) {
     const uint32_t B = BS ? BS : cv.B, BB = B * B;
-    if constexpr (!TRI) {
+    uint32_t i;
+    float wx = 0.f, wy = 0.f, wz = 0.f;
+    if constexpr (OFS && TRI) {
+        const uint32_t x = tri_bits(f.x, wx), y = tri_bits(f.y, wy), z = tri_bits(f.z, wz);
+        i = index_of<BS>(x, y, z, offset);
+    } else if constexpr (OFS) {
+        i = index_of<BS>(__float_as_uint(floor_bits(f.x)), __float_as_uint(floor_bits(f.y)),
+                                __float_as_uint(floor_bits(f.z)), offset - (BB + B + 1u));
+    } else if constexpr (TRI) {
+        uint32_t x0, y0, z0;
+        tri_axis<BS>(f.x, cv.c, cv.Beff, cv.beff_magic, B, x0, wx);
+        tri_axis<BS>(f.y, cv.c, cv.Beff, cv.beff_magic, B, y0, wy);
+        tri_axis<BS>(f.z, cv.c, cv.Beff, cv.beff_magic, B, z0, wz);
+        i = (z0 * B + y0) * B + x0;
+    } else {
         uint32_t lx = cv.c + mod_beff<BS>(floor_u(f.x), cv.Beff, cv.beff_magic);
         uint32_t ly = cv.c + mod_beff<BS>(floor_u(f.y), cv.Beff, cv.beff_magic);
         uint32_t lz = cv.c + mod_beff<BS>(floor_u(f.z), cv.Beff, cv.beff_magic);
+        if constexpr (BS == 0) {
+            lx = lx > 0 ? lx : 1u;
+            ly = ly > 0 ? ly : 1u;
+            lz = lz > 0 ? lz : 1u;
+        }
+        i = ((lz - 1) * B + (ly - 1)) * B + (lx - 1);
+    }
+    if constexpr (!TRI) {
         if constexpr (!std::is_same<T, TwoU8>::value) {
-            return sample_corner<T, BS>(reinterpret_cast<const T *>(base), B, lx, ly, lz);
+            return sample_corner<T, BS>(reinterpret_cast<const T *>(base), B, i);
         } else {
             // two interleaved u8 channels, voxel i channel k at byte 2 i + k
-            if constexpr (BS == 0) {
-                lx = lx > 0 ? lx : 1u;
-                ly = ly > 0 ? ly : 1u;
-                lz = lz > 0 ? lz : 1u;
-            }
-            const uint32_t i0 = ((lz - 1) * B + (ly - 1)) * B + (lx - 1);
-            const uint32_t id[8] = {i0,      i0 + 1,      i0 + B,      i0 + B + 1,
-                                    i0 + BB, i0 + BB + 1, i0 + BB + B, i0 + BB + B + 1};
+            const uint32_t id[8] = {i, i + 1, i + B, i + B + 1, i + BB, i + BB + 1, i + BB + B, i + BB + B + 1};
             uint32_t s0 = 0, s1 = 0;
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
@@ -408,15 +464,9 @@ __device__ __forceinline__ typename SampleOf<T>::type sample_brick(const uint8_t
             return make_float2(div_const<2040u>(u2f(s0)), div_const<2040u>(u2f(s1)));
         }
     } else {
-        uint32_t x0, y0, z0;
-        float wx, wy, wz;
-        tri_axis<BS>(f.x, cv.c, cv.Beff, cv.beff_magic, B, x0, wx);
-        tri_axis<BS>(f.y, cv.c, cv.Beff, cv.beff_magic, B, y0, wy);
-        tri_axis<BS>(f.z, cv.c, cv.Beff, cv.beff_magic, B, z0, wz);
         if constexpr (!std::is_same<T, TwoU8>::value) {
-            return sample_trilinear<T, BS>(reinterpret_cast<const T *>(base), B, x0, y0, z0, wx, wy, wz);
+            return sample_trilinear<T, BS>(reinterpret_cast<const T *>(base), B, i, wx, wy, wz);
         } else {
-            const uint32_t i = (z0 * B + y0) * B + x0;
             const uint32_t id[8] = {i, i + 1, i + B, i + B + 1, i + BB, i + BB + 1, i + BB + B, i + BB + B + 1};
             uchar2 v[8];
 #pragma unroll
@@ -576,6 +626,7 @@ struct Ray {
     float t_margin;  // margin of t_run for the roundings of t (+inf: no runs)
     float t_run; // below this t the next sample surely lies in the current brick and level, before tfar
     uint32_t slvl;  // cache level of the brick to sample
+    uint32_t offset;  // its origin_offset (kTakesOffset)
     bool pend;   // the ray stands at a sample of a resident, visible brick
     Walk w;
     bool unm, dvr;
@@ -698,6 +749,7 @@ __device__ __forceinline__ bool ray_setup(const LevelTables &lt, const ViewParam
     r.t_margin = dot(dir, dir) >= 0.98f ? vp.run_margin * tfar : __int_as_float(0x7f800000);
     r.pend = false;
     r.slvl = r.lvl;
+    r.offset = 0u;
     r.t_run = 0.f;
     r.maxOp = r.dvr ? 0.f : vp.state[4 * i];
     return true;
@@ -725,6 +777,12 @@ __device__ __forceinline__ void composite(Ray &r, float4 col) {
         r.fc.z = fmad(col.z, rr, r.fc.z);
         r.fc.w = fmad(col.w, rr, r.fc.w);
     }
+}
+
+// The sampler of a ray: known to the kernels of kOneCorner and kOneTrilinear.
+template <Views V>
+__device__ __forceinline__ bool corner_sampler(const Ray &r) {
+    return V == Views::kOneCorner || (V != Views::kOneTrilinear && r.sampler == GC_SAMPLER_REFERENCE);
 }
 
 // The march loop (RayCasters.cu:122-188) in two halves, so that the lanes of a
@@ -761,9 +819,10 @@ __device__ __forceinline__ float run_bound(const LevelTables &lt, const Ray &r, 
 // or it stepped through an invisible or empty brick.
 // ONE: the view's visible bins are kept in shared memory (`visible`), else in
 // its parameters.
-template <bool TL, bool ONE, bool TWO>
+template <typename T, uint32_t BS, bool TL, int N, Views V>
 __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables &lt, const unsigned long long *visible,
                                          const uint32_t *two_rows, Ray &r) {
+    constexpr bool TWO = std::is_same<T, TwoU8>::value, ONE = V != Views::kSeveral;
     const ViewParams &vp = *r.vp;
     if (!((!r.dvr || r.fc.w < r.early) && r.t < r.tfar)) return false;
     const V3 np = norm_pos(r.pos);
@@ -811,7 +870,29 @@ __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables 
         r.t_run = 0.f;
     }
     r.pend = st == kMapped || st == kCoarser;
-    if (r.pend) return true;
+    if (r.pend) {
+        if constexpr (kTakesOffset<T, BS, true, N, ONE>) {
+            if (!kTakesOffset<T, BS, false, N, ONE> && corner_sampler<V>(r)) return true;
+            // The brick that holds the sample's voxel is q but for roundings at a face
+            // that the ray just crossed.  The next samples only move away from that
+            // face (every operation up to the voxel keeps their order), so one offset
+            // holds for the run; where it is another brick, for this sample alone.
+            const float bf = u2f(cv.Beff);  // nbf * bf is vvoxf, exactly
+            const uint32_t x = floor_u(p.x * (lt.nbf[r.lvl][0] * bf)) - q.x * cv.Beff;
+            const uint32_t y = floor_u(p.y * (lt.nbf[r.lvl][1] * bf)) - q.y * cv.Beff;
+            const uint32_t z = floor_u(p.z * (lt.nbf[r.lvl][2] * bf)) - q.z * cv.Beff;
+            if (st == kMapped && max(max(x, y), z) < cv.Beff) {
+                r.offset = origin_offset<BS>(cv, q.x, q.y, q.z);
+            } else {
+                const uint32_t l = r.slvl, d = cv.beff_magic;
+                r.offset = origin_offset<BS>(cv, __umulhi(floor_u(np.x * lt.ior[l][0] * lt.vvoxf[l][0]), d),
+                                             __umulhi(floor_u(np.y * lt.ior[l][1] * lt.vvoxf[l][1]), d),
+                                             __umulhi(floor_u(np.z * lt.ior[l][2] * lt.vvoxf[l][2]), d));
+                r.t_run = 0.f;
+            }
+        }
+        return true;
+    }
     // Not sampled: the step of a sample whose opacity stays below 0.001 in an
     // invisible brick, the base step in an empty one (bare steps through it
     // only where they are no shorter than the level's, which t_run allows for)
@@ -840,7 +921,7 @@ __device__ __forceinline__ bool ray_walk(const CacheView &cv, const LevelTables 
 }
 
 // N samples at the positions pos[0 .. N-1] in the brick the ray stands in.
-template <typename T, uint32_t BS, bool TRI, int N>
+template <typename T, uint32_t BS, bool TRI, int N, bool OFS>
 __device__ __forceinline__ void take_samples(const CacheView &cv, const LevelTables &lt, const Ray &r,
                                              const V3 (&pos)[N + 1], typename SampleOf<T>::type (&out)[N]) {
     const uint32_t l = r.slvl;
@@ -849,22 +930,22 @@ __device__ __forceinline__ void take_samples(const CacheView &cv, const LevelTab
         const V3 np = norm_pos(pos[k]);
         const V3 p = v3(np.x * lt.ior[l][0], np.y * lt.ior[l][1], np.z * lt.ior[l][2]);
         const V3 f = v3(p.x * lt.vvoxf[l][0], p.y * lt.vvoxf[l][1], p.z * lt.vvoxf[l][2]);
-        out[k] = sample_brick<T, BS, TRI>(r.w.base, cv, f);
+        out[k] = sample_brick<T, BS, TRI, OFS>(r.w.base, cv, f, r.offset);
     }
 }
-template <typename T, uint32_t BS, bool TRI, int N>
+template <typename T, uint32_t BS, bool TRI, int N, bool OFS>
 __device__ __forceinline__ void take_samples_of(const CacheView &cv, const LevelTables &lt, const Ray &r,
                                                 const V3 (&pos)[N + 1], typename SampleOf<T>::type (&out)[N]) {
     if constexpr (std::is_same<T, MixedVoxel>::value) {
         const uint32_t eb = r.vp->eb;
         if (eb == 1)
-            take_samples<uint8_t, BS, TRI, N>(cv, lt, r, pos, out);
+            take_samples<uint8_t, BS, TRI, N, OFS>(cv, lt, r, pos, out);
         else if (eb == 2)
-            take_samples<uint16_t, BS, TRI, N>(cv, lt, r, pos, out);
+            take_samples<uint16_t, BS, TRI, N, OFS>(cv, lt, r, pos, out);
         else
-            take_samples<float, BS, TRI, N>(cv, lt, r, pos, out);
+            take_samples<float, BS, TRI, N, OFS>(cv, lt, r, pos, out);
     } else {
-        take_samples<T, BS, TRI, N>(cv, lt, r, pos, out);
+        take_samples<T, BS, TRI, N, OFS>(cv, lt, r, pos, out);
     }
 }
 
@@ -877,18 +958,19 @@ __device__ __forceinline__ void take_samples_of(const CacheView &cv, const Level
 // Per frame, one sample at a time -> these kernels: 512^2 with few rays 511 ->
 // 336 us, 1024^2 of a 512^3 u16 volume 3.15 -> 2.73 ms, trilinear maximum
 // intensity 5.55 -> 5.32 ms.
-template <typename T, uint32_t BS, int N, bool ONE>
+template <typename T, uint32_t BS, int N, Views V>
 __device__ __forceinline__ void ray_sample(const CacheView &cv, const LevelTables &lt, const float4 *pairs, Ray &r) {
+    constexpr bool ONE = V != Views::kSeveral;
     const ViewParams &vp = *r.vp;
     V3 pos[N + 1];
     pos[0] = r.pos;
 #pragma unroll
     for (int k = 0; k < N; ++k) pos[k + 1] = fma3(r.dir, r.step, pos[k]);
     typename SampleOf<T>::type sample[N];
-    if (r.sampler == GC_SAMPLER_REFERENCE)
-        take_samples_of<T, BS, false, N>(cv, lt, r, pos, sample);
+    if (corner_sampler<V>(r))
+        take_samples_of<T, BS, false, N, kTakesOffset<T, BS, false, N, ONE>>(cv, lt, r, pos, sample);
     else
-        take_samples_of<T, BS, true, N>(cv, lt, r, pos, sample);
+        take_samples_of<T, BS, true, N, kTakesOffset<T, BS, true, N, ONE>>(cv, lt, r, pos, sample);
     bool go = true;
     if (r.dvr) {
         float4 col[N];
@@ -933,15 +1015,15 @@ __device__ __forceinline__ void ray_sample(const CacheView &cv, const LevelTable
 // One round of a warp's rays: the lanes that must find their next brick walk,
 // then the lanes that stand at a sample take it.  Returns true when the lane's
 // ray ended.
-template <typename T, uint32_t BS, bool TL, int N, bool ONE>
+template <typename T, uint32_t BS, bool TL, int N, Views V>
 __device__ __forceinline__ bool ray_round(const CacheView &cv, const LevelTables &lt,
                                           const unsigned long long *visible, const uint32_t *two_rows,
                                           const float4 *pairs, Ray &r,
                                           bool active) {
     bool ended = false;
-    if (active && !r.pend) ended = !ray_walk<TL, ONE, std::is_same<T, TwoU8>::value>(cv, lt, visible, two_rows, r);
+    if (active && !r.pend) ended = !ray_walk<T, BS, TL, N, V>(cv, lt, visible, two_rows, r);
     __syncwarp();
-    if (active && r.pend) ray_sample<T, BS, N, ONE>(cv, lt, pairs, r);
+    if (active && r.pend) ray_sample<T, BS, N, V>(cv, lt, pairs, r);
     __syncwarp();
     return ended;
 }
@@ -1052,11 +1134,12 @@ __device__ __forceinline__ void retire_warp(uint32_t *queue, uint32_t nwarps) {
 // its own number and a launch whose tiles all are first tiles never touches the
 // queue.  A 128^2 frame: 99 -> 93 us; 777x555, two channels: 2.14 -> 2.05 ms.
 constexpr uint32_t kWideWarps = 24;
-template <typename T, uint32_t BS, bool TL, int N, bool ONE>
+template <typename T, uint32_t BS, bool TL, int N, Views V>
 __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
     render_kernel(const CacheView cv, const LevelTables lt, const __grid_constant__ ViewParams one,
                   const ViewParams *__restrict__ views, uint32_t nviews, uint32_t total_tiles, uint32_t *queue,
                   uint32_t nwarps) {
+    constexpr bool ONE = V != Views::kSeveral;
     __shared__ unsigned long long s_visible, s_samples[8], s_rays[8];  // of each warp
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (lane == 0) s_samples[warp] = s_rays[warp] = 0;
@@ -1087,7 +1170,7 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
         bool active = x < vp->W && y < vp->H && ray_setup<T>(lt, vp, x, y, r);
         if (active) marched = ray_enters(r);
         while (__any_sync(0xffffffffu, active)) {
-            if (ray_round<T, BS, TL, N, ONE>(cv, lt, &s_visible, s_two, s_pairs, r, active)) {
+            if (ray_round<T, BS, TL, N, V>(cv, lt, &s_visible, s_two, s_pairs, r, active)) {
                 active = false;
                 unm = ray_finish(r);
                 coarse_any = r.coarse;
@@ -1118,31 +1201,32 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
 // Kernel of a voxel kind (1, 2, 4 bytes, 0 mixed, kTwoChannelU8), brick size
 // (16 and 32 compiled for their size, others at run time) and samples at a
 // time; TL: for a two-level page directory.
-template <uint32_t BS, bool TL, int N, bool ONE>
+template <uint32_t BS, bool TL, int N, Views V>
 void *march_kernel_bs(uint32_t kind) {
     switch (kind) {
-        case 1: return reinterpret_cast<void *>(render_kernel<uint8_t, BS, TL, N, ONE>);
-        case 2: return reinterpret_cast<void *>(render_kernel<uint16_t, BS, TL, N, ONE>);
-        case 4: return reinterpret_cast<void *>(render_kernel<float, BS, TL, N, ONE>);
-        case 0: return reinterpret_cast<void *>(render_kernel<MixedVoxel, BS, TL, N, ONE>);
+        case 1: return reinterpret_cast<void *>(render_kernel<uint8_t, BS, TL, N, V>);
+        case 2: return reinterpret_cast<void *>(render_kernel<uint16_t, BS, TL, N, V>);
+        case 4: return reinterpret_cast<void *>(render_kernel<float, BS, TL, N, V>);
+        case 0: return reinterpret_cast<void *>(render_kernel<MixedVoxel, BS, TL, N, V>);
         // (two channels hold twice the values a sample)
-        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N < 4 ? N : 4, ONE>);
+        case 0x202: return reinterpret_cast<void *>(render_kernel<TwoU8, BS, TL, N < 4 ? N : 4, V>);
         default: return nullptr;
     }
 }
-template <int N, bool ONE>
+template <int N, Views V>
 void *march_kernel_n(uint32_t kind, uint32_t brick_size, bool two_level) {
     if (two_level)
-        return brick_size == 16 ? march_kernel_bs<16, true, N, ONE>(kind) : march_kernel_bs<0, true, N, ONE>(kind);
-    if (brick_size == 16) return march_kernel_bs<16, false, N, ONE>(kind);
-    if (brick_size == 32) return march_kernel_bs<32, false, N, ONE>(kind);
-    return march_kernel_bs<0, false, N, ONE>(kind);
+        return brick_size == 16 ? march_kernel_bs<16, true, N, V>(kind) : march_kernel_bs<0, true, N, V>(kind);
+    if (brick_size == 16) return march_kernel_bs<16, false, N, V>(kind);
+    if (brick_size == 32) return march_kernel_bs<32, false, N, V>(kind);
+    return march_kernel_bs<0, false, N, V>(kind);
 }
 void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShape shape) {
     switch (shape) {
-        case MarchShape::kOneFew: return march_kernel_n<6, true>(kind, brick_size, two_level);
-        case MarchShape::kOneMany: return march_kernel_n<2, true>(kind, brick_size, two_level);
-        default: return march_kernel_n<2, false>(kind, brick_size, two_level);
+        case MarchShape::kOneFew: return march_kernel_n<6, Views::kOne>(kind, brick_size, two_level);
+        case MarchShape::kOneMany: return march_kernel_n<2, Views::kOneCorner>(kind, brick_size, two_level);
+        case MarchShape::kOneManyTrilinear: return march_kernel_n<2, Views::kOneTrilinear>(kind, brick_size, two_level);
+        default: return march_kernel_n<2, Views::kSeveral>(kind, brick_size, two_level);
     }
 }
 
@@ -1232,7 +1316,7 @@ constexpr uint32_t kTwoChannelU8 = 0x202;
 static uint32_t voxel_kind(const CacheView &cv) { return cv.nc == 2 ? kTwoChannelU8 : cv.eb; }
 
 static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool two_level, uint32_t total_tiles,
-                                         uint32_t rect_tiles, bool one, bool long_rays) {
+                                         uint32_t rect_tiles, bool one, bool long_rays, bool trilinear) {
     const RenderTuning tune = render_tuning();
     const uint32_t threads = tune.threads;
     GC_REQUIRE(threads == 64 || threads == 128 || threads == 256, "render threads must be 64, 128 or 256");
@@ -1252,12 +1336,15 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
     // Launches of several views take the shape for many rays.
     const uint32_t few_warps = long_rays ? kWideWarps * 3u / 2u : kWideWarps;
     const bool few = one && rect_tiles <= static_cast<uint32_t>(sm_count()) * few_warps;
-    const MarchShape shape = few ? MarchShape::kOneFew : (one ? MarchShape::kOneMany : MarchShape::kSeveral);
+    const MarchShape shape = few          ? MarchShape::kOneFew
+                             : !one       ? MarchShape::kSeveral
+                             : trilinear  ? MarchShape::kOneManyTrilinear
+                                          : MarchShape::kOneMany;
     void *kernel = fast_build ? fast::march_kernel(eb, brick_size, two_level, shape)
                               : exact::march_kernel(eb, brick_size, two_level, shape);
     if (!kernel) fail(GC_ERR_UNSUPPORTED, "the ray caster supports one channel of 1, 2 or 4 bytes");
     const int slot = eb == 1 ? 0 : eb == 2 ? 1 : eb == 4 ? 2 : eb == 0 ? 3 : 4;
-    static int occupancy[2][3][5][3][5] = {};
+    static int occupancy[2][4][5][3][5] = {};
     const int tslot = threads == 64 ? 0 : (threads == 128 ? 1 : 2);
     const int bslot = two_level ? (brick_size == 16 ? 3 : 4) : (brick_size == 16 ? 0 : (brick_size == 32 ? 1 : 2));
     int &occ = occupancy[fast_build ? 1 : 0][static_cast<int>(shape)][slot][tslot][bslot];
@@ -1276,7 +1363,7 @@ static RenderLaunch render_launch_config(uint32_t eb, uint32_t brick_size, bool 
 void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev, uint32_t nviews,
                    uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
     ViewParams none{};
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), &none, &views_dev, &nviews,
@@ -1289,7 +1376,7 @@ void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewPar
                        uint32_t rect_tiles, uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
     const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, true,
-                                                view.mode == GC_MODE_DVR && cv.nc == 1);
+                                                view.mode == GC_MODE_DVR && cv.nc == 1, view.sampler != GC_SAMPLER_REFERENCE);
     uint32_t nwarps = L.grid * (L.threads / 32), nviews = 1;
     const ViewParams *views = nullptr;
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), const_cast<ViewParams *>(&view),
@@ -1319,7 +1406,7 @@ void launch_render_graph(RenderGraph &g, const CacheView &cv, const LevelTables 
                          const ViewParams *views_pinned, uint32_t nviews, uint32_t total_tiles, uint32_t rect_tiles,
                          uint32_t *queue, cudaStream_t s) {
     if (total_tiles == 0) return;
-    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false);
+    const RenderLaunch L = render_launch_config(voxel_kind(cv), cv.c ? cv.B : 0u, cv.pt.shift != 0u, total_tiles, rect_tiles, false, false, false);
     uint32_t nwarps = L.grid * (L.threads / 32);
     const ViewParams *vd = views_dev;
     ViewParams none{};
