@@ -722,8 +722,8 @@ def run_ours(args):
                            / measured_peak()[0], 3),
                        "value_bins_s": round(LAST_PREPROCESS.get("flags_bins_s", 0.0), 4),
                        "store_copy_s": round(LAST_PREPROCESS.get("copy_s", 0.0), 4),
-                       "note": "device mip pyramid (every level read once, every coarser level written: "
-                               "2 x pyramid - level 0 bytes, over the mip time); device bricking (every level "
+                       "note": "device mip pyramid (the volume read once, every coarser level written once, over "
+                               "the mip time); device bricking (every level "
                                "read once + the brick store written, over the bricking time; fraction of the "
                                "measured HBM peak); value bins of every brick; copy of the brick store to host "
                                "memory"},
