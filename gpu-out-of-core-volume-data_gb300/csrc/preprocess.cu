@@ -874,6 +874,8 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
     }
 }
 
+constexpr uint32_t kSlabShared = 200u << 10;  // shared memory of a slab's slices, at most
+
 // Launches the slab bricker where it applies: brick rows of whole 16- or 8-byte
 // chunks, a 16-byte aligned level, a store aligned to the chunks, and at least two
 // slices in shared memory.
@@ -898,7 +900,7 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
     sp.pitch = words * 16u;
     const uint32_t slice = p.B * sp.pitch;
     sp.stages = std::min(4u, (96u << 10) / slice);
-    if (sp.stages < 2u) sp.stages = std::min(2u, (200u << 10) / slice);
+    if (sp.stages < 2u) sp.stages = std::min(2u, kSlabShared / slice);
     if (sp.stages < 2u || p.B * sp.cprow >= 65536u) return false;
     const uint64_t slabs = static_cast<uint64_t>(sp.ngx) * (p.nbig[1] * p.BB[1]) * (p.nbig[2] * p.BB[2]);
     // at least four blocks per SM, as far as a slab has slices
@@ -914,8 +916,10 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
     const uint32_t grid = static_cast<uint32_t>(std::min<uint64_t>(sp.items, 1u << 30));
     const uint32_t bytes = sp.stages * slice;
     auto go = [&](auto kernel) {
+        // always to the same limit: the attribute belongs to the kernel, not to the
+        // call, and another thread's smaller slab must not lower it before this launch
         if (bytes > (48u << 10))
-            GC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
+            GC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabShared));
         kernel<<<grid, 256, bytes, s>>>(level, out, sp);
     };
     if (ch == 16)
