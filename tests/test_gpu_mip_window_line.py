@@ -33,7 +33,7 @@ def test_short_rows_above_the_line(gc, torch_cuda, eb, ch):
                                         (4, 1, True)])
 def test_sizes_beside_the_line(gc, torch_cuda, eb, ch, real):
     rng = np.random.default_rng(7 * eb + ch)
-    line = 16384 if eb == ch and ch > 1 else 49152
+    line = 28672 if eb == ch and ch > 1 else 49152
     for X in (3, 9, 17, 33, 67):
         chunks = (X // 2 * eb + 7) // 8
         for rows in (line // (chunks * 64) - 1, line // (chunks * 64), line // (chunks * 64) + 1):
