@@ -219,7 +219,7 @@ struct FrameScan {
     const uint32_t *usage[2];
     uint32_t nslots[2];        // 0: not counted
     uint32_t *count[2];        // results (device)
-    uint64_t *status;          // a word per scan tile, zero between launches
+    uint64_t *status;          // scan_status_words, zero between launches
     ScanCtl *ctl;
     uint32_t silent_tile;      // a tile that publishes nothing (tests of the error path; 0xffffffff: none)
     uint32_t scan_tiles, count_blocks[2];  // set by launch_frame_scan
@@ -237,8 +237,8 @@ constexpr uint32_t kClusterSlots = 131072;
 void launch_lru_cluster(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
                         uint32_t nslots, uint32_t *count, cudaStream_t s);
 // Status words of the two kernels for n items.
-uint32_t lru_tiles(uint64_t n);
-uint32_t scan_tiles(uint64_t n);
+uint32_t lru_status_words(uint64_t n);
+uint32_t scan_status_words(uint64_t n);
 
 struct InstallArgs {
     uint4 *mrpd;

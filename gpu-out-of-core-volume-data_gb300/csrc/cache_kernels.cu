@@ -40,9 +40,24 @@ constexpr uint32_t kMaxSpins = 1u << 22;
 constexpr uint32_t kLruItems = 16, kLruTile = kThreads * kLruItems;
 constexpr uint32_t kScanWords = 8, kScanTile = kThreads * kScanWords * 4;
 
-// A tile's status word: the published bit, then its count.  The word is all that
-// is handed over, so relaxed accesses do (no other memory is ordered by it).
+// A tile's status word: the published bit, then its count.  In a scan of more than
+// a number of tiles (kScanGrouped, kLruGrouped) the words are followed by one per
+// whole group of kGroup tiles, with the group's sum, which its last tile publishes.
+// The words are all that is handed over, so relaxed accesses do (no other memory
+// is ordered by them).
+//
+// With groups a tile reads at most 256 words and one per 256 tiles, without them
+// one per tile before it, which grows with the square of the tiles; but a sum
+// comes a hop later.  Request scan: 6.4 M entries (782 tiles), misses in most,
+// 19.7 us without, 17.4 with groups; update of a 403 M entry directory (49,297
+// tiles) with 10,000 misses / a miss in every tile 589 / 1,549 -> 447 / 688 us.
+// LRU update, every tile of which waits: 8,192 tiles 220 us without, 247 with
+// groups; 16,384 487 / 466; 32,768 1,254 / 910.
 constexpr uint64_t kPublished = 1ull << 32;
+constexpr uint32_t kGroup = 256, kScanGrouped = 256, kLruGrouped = 12288;
+__host__ __device__ constexpr uint32_t whole_groups(uint32_t tiles, uint32_t grouped) {
+    return tiles > grouped ? tiles / kGroup : 0u;
+}
 __device__ __forceinline__ void publish(uint64_t *status, uint32_t count) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(status), "l"(kPublished | count) : "memory");
 }
@@ -64,25 +79,46 @@ __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *s_warp) {
     return t;
 }
 
-// The number of flagged items in the tiles before `tile`, whose count this
-// tile's block has published: each thread waits (bounded) for the counts of
-// some predecessors, so that no tile waits for a chain of others.  Tiles are
-// handed out by a ticket, so every predecessor's block has started.
-__device__ uint32_t predecessors(const uint64_t *status, uint32_t tile, uint32_t *err, uint32_t *s_warp) {
+// This thread's share of the sum of n published words, each waited for (bounded).
+__device__ __forceinline__ uint32_t published(const uint64_t *words, uint32_t n, uint32_t *err) {
     uint32_t sum = 0, spins = 0;
 #pragma unroll 4
-    for (uint32_t j = threadIdx.x; j < tile; j += kThreads) {
-        uint64_t v = status_of(status + j);
+    for (uint32_t j = threadIdx.x; j < n; j += kThreads) {
+        uint64_t v = status_of(words + j);
         while (!(v & kPublished)) {
             if (++spins > kMaxSpins) {
                 atomicOr(err, kErrLookback);
                 break;
             }
             __nanosleep(32);
-            v = status_of(status + j);
+            v = status_of(words + j);
         }
         sum += static_cast<uint32_t>(v);
     }
+    return sum;
+}
+
+// True for the tiles that publish their group's sum, and so call predecessors.
+__device__ __forceinline__ bool ends_group(uint32_t tile, uint32_t groups) {
+    return tile < groups * kGroup && tile % kGroup == kGroup - 1u;
+}
+
+// The number of flagged items in the tiles before `tile`, whose count `total` this
+// tile's block has published: the threads wait for the tiles before it (in its
+// group, and for the whole groups before that, where the scan has groups), so that
+// no tile waits for a chain of others.  Tiles are handed out by a ticket, so every
+// predecessor's block has started.
+// only_group: the tile has nothing flagged and wants no sum.
+__device__ uint32_t predecessors(uint64_t *status, uint32_t tile, uint32_t tiles, uint32_t groups, uint32_t total,
+                                 bool only_group, uint32_t *err, uint32_t *s_warp) {
+    const uint32_t group = groups ? tile / kGroup : 0u, first = group * kGroup;
+    uint32_t sum = published(status + first, tile - first, err);
+    if (ends_group(tile, groups)) {
+        const uint32_t in_group = block_sum(sum, s_warp);
+        if (threadIdx.x == 0) publish(status + tiles + group, in_group + total);
+    }
+    if (only_group) return 0;
+    sum += published(status + tiles, group, err);
     return block_sum(sum, s_warp);
 }
 
@@ -129,7 +165,8 @@ __global__ void __launch_bounds__(kThreads) lru_partition_kernel(const uint32_t 
         total += s_used[w];
     }
     if (threadIdx.x == 0) publish(status + tile, total);
-    before += predecessors(status, tile, &ctl->err, s_warp);
+    const uint32_t groups = whole_groups(gridDim.x, kLruGrouped);
+    before += predecessors(status, tile, gridDim.x, groups, total, false, &ctl->err, s_warp);
     const uint32_t total_used = *count;
     bool bad = false;
 #pragma unroll
@@ -148,7 +185,7 @@ __global__ void __launch_bounds__(kThreads) lru_partition_kernel(const uint32_t 
     }
     if (bad) atomicOr(&ctl->err, kErrLookback);
     if (ends_launch(ctl)) {
-        for (uint32_t j = threadIdx.x; j < gridDim.x; j += kThreads) status[j] = 0;
+        for (uint32_t j = threadIdx.x; j < gridDim.x + groups; j += kThreads) status[j] = 0;
         if (threadIdx.x == 0) ctl->ticket = ctl->done = 0;
     }
 }
@@ -230,6 +267,7 @@ __global__ void __launch_bounds__(kThreads) frame_scan_kernel(const FrameScan a,
     __shared__ uint32_t s_tile, s_warp[kWarps], s_used[kWarps];
     __shared__ uint16_t s_entry[kScanTile];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t groups = whole_groups(a.scan_tiles, kScanGrouped);
     if (blockIdx.x < a.scan_tiles) {
         if (threadIdx.x == 0) s_tile = atomicAdd(&a.ctl->ticket, 1u);
         __syncthreads();
@@ -280,13 +318,16 @@ __global__ void __launch_bounds__(kThreads) frame_scan_kernel(const FrameScan a,
                         if ((f >> k) & 1u)
                             s_entry[r++] = static_cast<uint16_t>(warp * (128u * kScanWords) + 128u * u + 4u * lane + k);
                 }
-                const uint32_t first = predecessors(a.status, tile, &a.ctl->err, s_warp);  // also a barrier
+                const uint32_t first =
+                    predecessors(a.status, tile, a.scan_tiles, groups, total, false, &a.ctl->err, s_warp);  // also a barrier
                 const uint32_t n = first < a.maxreq ? min(total, a.maxreq - first) : 0u;
                 for (uint32_t r = threadIdx.x; r < n; r += kThreads) {
                     const uint4 b = decode_request(tile * kScanTile + s_entry[r], a.mx, a.my, lt);
                     a.list[first + r] = b;
                     if (a.host_list) a.host_list[first + r] = b;
                 }
+            } else if (ends_group(tile, groups)) {
+                predecessors(a.status, tile, a.scan_tiles, groups, 0u, true, &a.ctl->err, s_warp);
             }
         }
     } else {
@@ -304,12 +345,14 @@ __global__ void __launch_bounds__(kThreads) frame_scan_kernel(const FrameScan a,
     // the last block: the totals, and everything as the next launch expects it
     uint32_t sum = 0;
     bool missing = false;
-    for (uint32_t j = threadIdx.x; j < a.scan_tiles; j += kThreads) {
+    const uint32_t in_groups = groups * kGroup;  // tiles summed by their groups
+    for (uint32_t j = in_groups + threadIdx.x; j < a.scan_tiles + groups; j += kThreads) {
         const uint64_t v = status_of(a.status + j);
         missing = missing || !(v & kPublished);
         sum += static_cast<uint32_t>(v);
         a.status[j] = 0;
     }
+    for (uint32_t j = threadIdx.x; j < in_groups; j += kThreads) a.status[j] = 0;
     missing = __syncthreads_or(missing);
     sum = block_sum(sum, s_warp);
     if (threadIdx.x == 0) {
@@ -859,8 +902,10 @@ __global__ void __launch_bounds__(256) completude_kernel(const float4 *__restric
 }
 
 // ---------------------------------------------------------------------------
-uint32_t lru_tiles(uint64_t n) { return static_cast<uint32_t>((n + kLruTile - 1) / kLruTile); }
-uint32_t scan_tiles(uint64_t n) { return static_cast<uint32_t>((n + kScanTile - 1) / kScanTile); }
+static uint32_t lru_tiles(uint64_t n) { return static_cast<uint32_t>((n + kLruTile - 1) / kLruTile); }
+static uint32_t scan_tiles(uint64_t n) { return static_cast<uint32_t>((n + kScanTile - 1) / kScanTile); }
+uint32_t lru_status_words(uint64_t n) { return lru_tiles(n) + whole_groups(lru_tiles(n), kLruGrouped); }
+uint32_t scan_status_words(uint64_t n) { return scan_tiles(n) + whole_groups(scan_tiles(n), kScanGrouped); }
 
 void launch_frame_scan(FrameScan a, const LevelTables &lt, cudaStream_t s) {
     a.scan_tiles = a.nscan ? scan_tiles(a.nscan) : 0u;
@@ -1175,7 +1220,8 @@ void launch_completude(const float4 *slot_vpos, uint32_t nslots, uint32_t *count
 // frame deadline that must not block in the allocator (cudaMalloc can wait for
 // the device), or a plug-in whose host application owns every byte of device
 // memory and hands it only input and output buffers.  For them the scan's
-// scratch -- one status word per 8192-entry tile and the scan control block -- lives in this file-scope device array instead of memory
+// scratch -- a status word per 8192-entry tile and per 256 tiles and the scan
+// control block -- lives in this file-scope device array instead of memory
 // obtained from cudaMalloc.  Every GPU that loads the library holds it until
 // the process exits.
 namespace gc {
@@ -1183,10 +1229,11 @@ namespace gc {
 constexpr uint32_t kNoAllocMaxTiles = 1024;  // request buffers of up to 1024 * 8192 entries
 constexpr uint64_t kNoAllocMaxEntries = static_cast<uint64_t>(kNoAllocMaxTiles) * kScanTile;
 
-// ScanCtl, then a status word per tile
-constexpr uint32_t kNoAllocWords = kNoAllocMaxTiles + sizeof(ScanCtl) / sizeof(uint64_t);
+// ScanCtl, then the status words
+constexpr uint32_t kNoAllocWords =
+    kNoAllocMaxTiles + whole_groups(kNoAllocMaxTiles, kScanGrouped) + sizeof(ScanCtl) / sizeof(uint64_t);
 static_assert(sizeof(ScanCtl) % sizeof(uint64_t) == 0, "ScanCtl must fill whole scratch words");
-static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];  // 8 KiB + 32 B
+static __device__ __align__(256) uint64_t g_noalloc_scratch[kNoAllocWords];  // 8 KiB + 64 B
 
 // Host code cannot use g_noalloc_scratch as a device address (the name is a
 // host-side stand-in); the device address is looked up once per device, with
@@ -1252,7 +1299,7 @@ extern "C" int gc_miss_list_noalloc(const uint32_t *requests, uint64_t n_entries
         uint64_t *status = reinterpret_cast<uint64_t *>(ctl + 1);
         // The scan leaves the scratch as it found it, but calls that overlapped (see
         // the header) may not have: every call starts from zeros.
-        GC_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ScanCtl) + scan_tiles(n_entries - 1) * sizeof(uint64_t), s));
+        GC_CUDA(cudaMemsetAsync(ctl, 0, sizeof(ScanCtl) + scan_status_words(n_entries - 1) * sizeof(uint64_t), s));
         FrameScan a{};
         a.req = requests;
         a.nscan = n_entries - 1;

@@ -1138,13 +1138,13 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
             C->pt_word_of = dalloc<uint32_t>(maxr, "page-table claim words");
             C->pt_jobs = dalloc<uint2>(maxr, "page-table jobs");
             C->pt_njobs = dalloc<uint32_t>(1, "page-table job count");
-            C->status_pt = dalloc<uint64_t>(lru_tiles(C->pt_slots), "scan status");
+            C->status_pt = dalloc<uint64_t>(lru_status_words(C->pt_slots), "scan status");
             C->ctl_pt = dalloc<ScanCtl>(1, "scan control");
             GC_CUDA(cudaMemset(C->pt.top, 0, C->pt_words * sizeof(uint32_t)));
             GC_CUDA(cudaMemset(C->pt.table, 0, C->pt_slots * per * sizeof(uint4)));
             GC_CUDA(cudaMemset(C->pt.usage, 0, C->pt_slots * sizeof(uint32_t)));
             GC_CUDA(cudaMemset(C->pt_claim, 0xff, C->pt_words * sizeof(uint32_t)));
-            GC_CUDA(cudaMemset(C->status_pt, 0, lru_tiles(C->pt_slots) * sizeof(uint64_t)));
+            GC_CUDA(cudaMemset(C->status_pt, 0, lru_status_words(C->pt_slots) * sizeof(uint64_t)));
             GC_CUDA(cudaMemset(C->ctl_pt, 0, sizeof(ScanCtl)));
             launch_pt_init(C->pt_order[0], C->pt_keys, C->pt_slots, nullptr);
         } else {
@@ -1167,8 +1167,8 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
         C->d_samples = dalloc<unsigned long long>(2, "sample and ray counters");
         GC_CUDA(cudaMemset(C->d_samples, 0, 2 * sizeof(unsigned long long)));
         GC_CUDA(cudaMemset(C->slot_bins, 0xff, C->nslots * sizeof(unsigned long long)));
-        C->status_lru = dalloc<uint64_t>(lru_tiles(C->nslots), "scan status");
-        C->status_miss = dalloc<uint64_t>(scan_tiles(C->nentries), "scan status");
+        C->status_lru = dalloc<uint64_t>(lru_status_words(C->nslots), "scan status");
+        C->status_miss = dalloc<uint64_t>(scan_status_words(C->nentries), "scan status");
         C->ctl_lru = dalloc<ScanCtl>(1, "scan control");
         C->ctl_miss = dalloc<ScanCtl>(1, "scan control");
         C->d_count = dalloc<uint32_t>(1, "counter");
@@ -1199,8 +1199,8 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
         GC_CUDA(cudaMemset(C->req, 0, C->nentries * sizeof(uint32_t)));
         GC_CUDA(cudaMemset(C->usage, 0, C->nslots * sizeof(uint32_t)));
         GC_CUDA(cudaMemset(C->pool, 0, C->nslots * C->slot_bytes));
-        GC_CUDA(cudaMemset(C->status_lru, 0, lru_tiles(C->nslots) * sizeof(uint64_t)));
-        GC_CUDA(cudaMemset(C->status_miss, 0, scan_tiles(C->nentries) * sizeof(uint64_t)));
+        GC_CUDA(cudaMemset(C->status_lru, 0, lru_status_words(C->nslots) * sizeof(uint64_t)));
+        GC_CUDA(cudaMemset(C->status_miss, 0, scan_status_words(C->nentries) * sizeof(uint64_t)));
         GC_CUDA(cudaMemset(C->ctl_lru, 0, sizeof(ScanCtl)));
         GC_CUDA(cudaMemset(C->ctl_miss, 0, sizeof(ScanCtl)));
         GC_CUDA(cudaMemset(C->d_queue, 0, 4 * sizeof(uint32_t)));
