@@ -69,3 +69,21 @@ def test_lru_order_at_group_edges(gc, torch_cuda, n):
         assert cm.stats().last_used == used.sum()
     assert cm.stats().device_error == 0
     cm.close()
+
+
+@pytest.mark.parametrize("n", [131073, 131074, 131075, 131076, 2490368, 2490371])
+def test_used_slots_of_any_remainder(gc, torch_cuda, n):
+    """The used slots of pools above one cluster, counted four at a time."""
+    vol = gc.volume_desc((64, 64, 64), 4, 1, 1)
+    cm = gc.CacheManager(vol, gc.compute_layout(vol), (n, 1, 1), max_requests=1)
+    cm.set_source_callback(lambda *a: gc.BRICK_UNKNOWN)
+    rng = np.random.default_rng(n)
+    for used in ([], [0], [n - 1], [n - 2, n - 3], rng.choice(n, 1000, replace=False), np.arange(n)):
+        ts = cm.timestamp()
+        usage = np.full(n, ts + 1, np.uint32)
+        usage[np.asarray(used, np.int64)] = ts
+        cm.load_buffer(gc.DUMP_USAGE, usage)
+        cm.update()
+        assert cm.stats().last_used == len(used)
+    assert cm.stats().device_error == 0
+    cm.close()
