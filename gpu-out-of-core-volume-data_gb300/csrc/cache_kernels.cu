@@ -1262,7 +1262,8 @@ static uint64_t *g_noalloc_ptr[kNoAllocMaxDevices] = {};
 static std::mutex g_noalloc_mu;
 
 // Test hook of the error path: GC_TEST_NOALLOC_SILENT_TILE=<k> makes scan tile
-// k publish nothing, so that tile k + 1's bounded look-back wait runs out.
+// k publish nothing, so that the bounded waits of the later tiles with flagged
+// entries run out (or, with none, the end of the launch finds the word missing).
 static uint32_t noalloc_silent_tile() {
     const char *v = std::getenv("GC_TEST_NOALLOC_SILENT_TILE");
     return (v && *v) ? static_cast<uint32_t>(std::strtoul(v, nullptr, 10)) : 0xffffffffu;
