@@ -1006,48 +1006,84 @@ __global__ void __launch_bounds__(256) empty_kernel(const uint8_t *__restrict__ 
     }
 }
 
-// The same for big bricks of whole 16-byte chunks, 16-byte aligned: G threads per
-// big brick, 16 bytes a lane with four loads in flight, ended by a vote once a
-// value reaches the threshold (an integer brick is empty when its largest value
-// is below it).  Bound by the read of the bricks that are empty; the first turn
-// (2 KiB with a warp, 16 KiB with a block) is read of every brick.  A warp per
-// big brick below 32 KiB (the reads of a turn fit the brick), a block above.
-// The bricks of a 768^3 u16 volume (16^3, 1.36 GB): 712 -> 66 us.
+// One turn of G threads over a big brick, four 16-byte loads in flight a thread, from
+// chunk c0 on: true where a value of the thread's chunks reaches the threshold.
 template <int CB, int G>
-__global__ void __launch_bounds__(256) empty_vec_kernel(const uint4 *__restrict__ bricks, uint64_t nbig,
-                                                        uint64_t chunks, float threshold,
-                                                        uint8_t *__restrict__ flags) {
-    constexpr uint32_t kPer = 256 / G;
-    const uint32_t lane = threadIdx.x % G;
-    for (uint64_t b = static_cast<uint64_t>(blockIdx.x) * kPer + threadIdx.x / G; b < nbig;
-         b += static_cast<uint64_t>(gridDim.x) * kPer) {
+__device__ __forceinline__ bool reaches(const uint4 *__restrict__ p, uint64_t c0, uint32_t lane, uint64_t chunks,
+                                        float threshold) {
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const uint64_t c = c0 + u * G + lane;
+        if (c < chunks) v[u] = __ldcs(p + c);
+    }
+    ValueRange<CB> range;
+    bool over = false, any = false;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (c0 + u * G + lane < chunks) {
+            any = true;
+            if constexpr (CB == 4) {
+                over = over || !(__uint_as_float(v[u].x) < threshold) || !(__uint_as_float(v[u].y) < threshold) ||
+                       !(__uint_as_float(v[u].z) < threshold) || !(__uint_as_float(v[u].w) < threshold);
+            } else {
+                range.add(v[u]);
+            }
+        }
+    }
+    if constexpr (CB != 4) over = any && !(static_cast<float>(range.highest()) < threshold);
+    return over;
+}
+
+// The same for big bricks of whole 16-byte chunks, 16-byte aligned, a warp each, 16
+// bytes a lane with four loads in flight, ended by a vote once a value reaches the
+// threshold (an integer brick is empty when its largest value is below it).  Bound
+// by the read of the bricks that are empty; the first 2 KiB are read of every
+// brick.  The bricks of a 768^3 u16 volume (16^3, 1.36 GB): 712 -> 66 us; 16,384 big
+// bricks of 32 KiB dense / half of them empty / all empty, value by value 13 / 450 /
+// 777, a block each 42 / 61 / 77, a warp each 9 / 56 / 87 us.
+template <int CB>
+__global__ void __launch_bounds__(256) empty_warp_kernel(const uint4 *__restrict__ bricks, uint64_t nbig,
+                                                         uint64_t chunks, float threshold,
+                                                         uint8_t *__restrict__ flags) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t b = static_cast<uint64_t>(blockIdx.x) * 8u + threadIdx.x / 32u; b < nbig;
+         b += static_cast<uint64_t>(gridDim.x) * 8u) {
         const uint4 *p = bricks + b * chunks;
         bool nonempty = false;
-        for (uint64_t c0 = 0; c0 < chunks && !nonempty; c0 += 4u * G) {
-            uint4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const uint64_t c = c0 + u * G + lane;
-                if (c < chunks) v[u] = __ldcs(p + c);
-            }
-            ValueRange<CB> range;
-            bool over = false, any = false;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (c0 + u * G + lane < chunks) {
-                    any = true;
-                    if constexpr (CB == 4) {
-                        over = over || !(__uint_as_float(v[u].x) < threshold) || !(__uint_as_float(v[u].y) < threshold) ||
-                               !(__uint_as_float(v[u].z) < threshold) || !(__uint_as_float(v[u].w) < threshold);
-                    } else {
-                        range.add(v[u]);
-                    }
-                }
-            }
-            if constexpr (CB != 4) over = any && !(static_cast<float>(range.highest()) < threshold);
-            nonempty = G == 256 ? __syncthreads_or(over) != 0 : __any_sync(0xffffffffu, over) != 0;
-        }
+        for (uint64_t c0 = 0; c0 < chunks && !nonempty; c0 += 128u)
+            nonempty = __any_sync(0xffffffffu, reaches<CB, 32>(p, c0, lane, chunks, threshold)) != 0;
         if (lane == 0) flags[b] = nonempty ? 0 : 1;
+    }
+}
+
+// Big bricks of 32 KiB and more that are no warps enough: a block takes `per` of them
+// (up to 8, as far as the bricks fill the SMs), a warp first looks at the first 512
+// bytes of each, and the whole block reads those that this leaves open.  4,854 big
+// bricks of 108 KiB dense / half of them empty / all empty, value by value 6.6 / 433 /
+// 760, a block each without the look (16 KiB of every brick) 15 / 46 / 79, with it 5.5 /
+// 46 / 82 us; 1,024 of 32 KiB 4.5 / 27 / 27, 5.7 / 6.5 / 6.8, 4.4 / 6.8 / 8.5 us.
+template <int CB>
+__global__ void __launch_bounds__(256) empty_block_kernel(const uint4 *__restrict__ bricks, uint64_t nbig,
+                                                          uint64_t chunks, uint32_t per, float threshold,
+                                                          uint8_t *__restrict__ flags) {
+    __shared__ uint32_t s_open[8];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * per;
+    bool open = false;
+    if (warp < per && b0 + warp < nbig) {
+        open = !__any_sync(0xffffffffu, reaches<CB, 32>(bricks + (b0 + warp) * chunks, 0, lane, 32, threshold));
+        if (!open && lane == 0) flags[b0 + warp] = 0;
+    }
+    if (lane == 0) s_open[warp] = open;
+    __syncthreads();
+    for (uint32_t w = 0; w < per; ++w) {
+        if (!s_open[w]) continue;  // the same for the block
+        const uint4 *p = bricks + (b0 + w) * chunks;
+        bool nonempty = false;
+        for (uint64_t c0 = 0; c0 < chunks && !nonempty; c0 += 1024u)
+            nonempty = __syncthreads_or(reaches<CB, 256>(p, c0, tid, chunks, threshold)) != 0;
+        if (tid == 0) flags[b0 + w] = nonempty ? 0 : 1;
     }
 }
 
@@ -1144,19 +1180,24 @@ int gc_bricks_empty(const void *bricks, uint64_t nb_big_bricks, const gc_volume_
         const uint32_t cb = channel_bytes(*vol);
         const uint64_t bytes = values * cb;
         if (bytes % 16 == 0 && reinterpret_cast<uintptr_t>(bricks) % 16 == 0 && (cb == 1 || cb == 2 || cb == 4)) {
-            const bool warp = bytes < (32u << 10);
-            const uint64_t blocks = std::min<uint64_t>(warp ? (nb_big_bricks + 7) / 8 : nb_big_bricks,
-                                                       static_cast<uint64_t>(sm_count()) * 64);
-            auto go = [&](auto kernel) {
-                kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
-                    static_cast<const uint4 *>(bricks), nb_big_bricks, bytes / 16, threshold, flags);
-            };
-            if (cb == 1)
-                warp ? go(empty_vec_kernel<1, 32>) : go(empty_vec_kernel<1, 256>);
-            else if (cb == 2)
-                warp ? go(empty_vec_kernel<2, 32>) : go(empty_vec_kernel<2, 256>);
-            else
-                warp ? go(empty_vec_kernel<4, 32>) : go(empty_vec_kernel<4, 256>);
+            const auto *in = static_cast<const uint4 *>(bricks);
+            const uint64_t sms = static_cast<uint64_t>(sm_count());
+            // a warp per big brick, above 32 KiB only where the bricks are warps enough
+            if (bytes < (32u << 10) || (bytes <= (128u << 10) && nb_big_bricks >= sms * 48)) {
+                const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((nb_big_bricks + 7) / 8, sms * 64));
+                auto go = [&](auto kernel) {
+                    kernel<<<blocks, 256, 0, as_stream(stream)>>>(in, nb_big_bricks, bytes / 16, threshold, flags);
+                };
+                cb == 1 ? go(empty_warp_kernel<1>) : cb == 2 ? go(empty_warp_kernel<2>) : go(empty_warp_kernel<4>);
+            } else {
+                const uint32_t per =
+                    static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(8, nb_big_bricks / (sms * 8))));
+                const unsigned blocks = static_cast<unsigned>((nb_big_bricks + per - 1) / per);
+                auto go = [&](auto kernel) {
+                    kernel<<<blocks, 256, 0, as_stream(stream)>>>(in, nb_big_bricks, bytes / 16, per, threshold, flags);
+                };
+                cb == 1 ? go(empty_block_kernel<1>) : cb == 2 ? go(empty_block_kernel<2>) : go(empty_block_kernel<4>);
+            }
             GC_CUDA(cudaGetLastError());
             count_launch();
             return;
