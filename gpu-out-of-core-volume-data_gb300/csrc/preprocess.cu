@@ -689,8 +689,8 @@ __device__ __forceinline__ void copies_wait(uint32_t left) {
 // a warp per run of bricks straight from the level (32-byte pieces of 16 bricks a
 // store) -> 347 us, 6.5 TB/s; its level of 8 bricks 51 -> 4.4 us; level 0 of a
 // 381x347x291 u8 volume (rows of odd length) 310 us voxel by voxel -> 25 us.
-template <int CH>
-__global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restrict__ level, uint8_t *__restrict__ out,
+template <int CH, uint32_t NT>
+__global__ void __launch_bounds__(NT) brick_slab_kernel(const uint8_t *__restrict__ level, uint8_t *__restrict__ out,
                                                          const SlabParams sp) {
     extern __shared__ __align__(128) uint8_t slab_smem[];
     const BrickParams &p = sp.p;
@@ -803,10 +803,10 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
         Chunk ck[kPre];
 #pragma unroll
         for (uint32_t u = 0; u < kPre; ++u) {
-            cp[u] = copy_of(min(tid + 256u * u, ncopy - 1u));
-            ck[u] = chunk_of(min(tid + 256u * u, nchunks - 1u));
+            cp[u] = copy_of(min(tid + NT * u, ncopy - 1u));
+            ck[u] = chunk_of(min(tid + NT * u, nchunks - 1u));
         }
-        if ((plane & 15) == 0 && ncopy <= 256u * kPre && nchunks <= 256u * kPre) {
+        if ((plane & 15) == 0 && ncopy <= NT * kPre && nchunks <= NT * kPre) {
             // Planes whole 16-byte chunks apart: a row starts at the same byte of its
             // first chunk in every slice, so a thread's copies and chunks only advance
             // by a plane and an output slice.
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
                     const bool z_in = z0 + i >= 0 && z0 + i < p.D[2];  // the same for the block
 #pragma unroll
                     for (uint32_t u = 0; u < kPre; ++u) {
-                        if (tid + 256u * u < ncopy) {
+                        if (tid + NT * u < ncopy) {
                             const uint32_t k = z_in ? n[u] : 0u;
                             copy16_async(smem + to_stage + cp[u].to, k ? src[u] : level, k);
                         }
@@ -844,7 +844,7 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
                 copy_slice(i + sp.stages - 1u);
 #pragma unroll
                 for (uint32_t u = 0; u < kPre; ++u) {
-                    if (tid + 256u * u < nchunks)
+                    if (tid + NT * u < nchunks)
                         put_bytes(slab_smem + from_stage + ck[u].row, ck[u].at, ck[u].zeros, ck[u].dst);
                     ck[u].dst += dslice;
                 }
@@ -856,8 +856,8 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
                     const uint32_t stage = smem + (i % sp.stages) * slice_bytes;
 #pragma unroll
                     for (uint32_t u = 0; u < kPre; ++u)
-                        if (tid + 256u * u < ncopy) copy_chunk(cp[u], i, stage);
-                    for (uint32_t t = tid + 256u * kPre; t < ncopy; t += 256u) copy_chunk(copy_of(t), i, stage);
+                        if (tid + NT * u < ncopy) copy_chunk(cp[u], i, stage);
+                    for (uint32_t t = tid + NT * kPre; t < ncopy; t += NT) copy_chunk(copy_of(t), i, stage);
                 }
                 copies_commit();
             };
@@ -869,8 +869,8 @@ __global__ void __launch_bounds__(256) brick_slab_kernel(const uint8_t *__restri
                 const uint8_t *stage = slab_smem + (i % sp.stages) * slice_bytes;
 #pragma unroll
                 for (uint32_t u = 0; u < kPre; ++u)
-                    if (tid + 256u * u < nchunks) put_chunk(ck[u], i, stage);
-                for (uint32_t t = tid + 256u * kPre; t < nchunks; t += 256u) put_chunk(chunk_of(t), i, stage);
+                    if (tid + NT * u < nchunks) put_chunk(ck[u], i, stage);
+                for (uint32_t t = tid + NT * kPre; t < nchunks; t += NT) put_chunk(chunk_of(t), i, stage);
             }
         }
         __syncthreads();  // the last slices have been read before the next slab's copies
@@ -890,9 +890,14 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
     sp.p = p;
     sp.cpr = row / ch;
     const uint32_t nsx = p.nbig[0] * p.BB[0];
-    // about 512 output chunks a slice (two per thread), at most 1 KiB of a row
-    sp.nb = std::max(1u, std::min(std::min(nsx, 512u / std::max(1u, p.B * sp.cpr)), 1024u / (p.Beff * p.eb)));
+    // about 512 output chunks a slice (two per thread), fewer of the smallest bricks,
+    // whose slabs have few slices; at most 1 KiB of a row, and of the smallest bricks
+    // no more than the copies of a slice are two per thread too
+    const uint32_t chunks = p.B <= 4 ? 128u : p.B <= 8 ? 256u : 512u;
+    const uint32_t in_row = p.B > 8 ? 1024u / (p.Beff * p.eb) : (16u * (chunks / p.B) - 15u - row) / (p.Beff * p.eb) + 1u;
+    sp.nb = std::max(1u, std::min(std::min(nsx, chunks / std::max(1u, p.B * sp.cpr)), in_row));
     sp.ngx = (nsx + sp.nb - 1) / sp.nb;
+    sp.nb = (nsx + sp.ngx - 1) / sp.ngx;  // slabs of about the same size
     const uint32_t span = (sp.nb - 1) * p.Beff * p.eb + row;
     sp.cprow = (15u + span + 15u) / 16u;
     // the lanes of a quarter warp read 16-byte words of rows a pitch apart: cpr
@@ -906,10 +911,18 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
     if (sp.stages < 2u) sp.stages = std::min(2u, kSlabShared / slice);
     if (sp.stages < 2u || p.B * sp.cprow >= 65536u) return false;
     const uint64_t slabs = static_cast<uint64_t>(sp.ngx) * (p.nbig[1] * p.BB[1]) * (p.nbig[2] * p.BB[2]);
-    // at least four blocks per SM, as far as a slab has slices
+    // two copies and two chunks a thread: blocks of 64 or 128 threads where those fill no
+    // more, so that more slabs are in flight.  Blocks of 256 / these: floats in 4^3
+    // bricks, covering 1, 64^3 12.8 / 7.2 us, 384^3 577 / 440 (a warp per run of bricks
+    // 8.3 and 596); u8 in 8^3 bricks 128^3 10.6 / 6.6, in 16^3 bricks 160^3 11.1 / 7.1
+    const uint32_t work = std::max(sp.nb * p.B * sp.cpr, p.B * sp.cprow);
+    const uint32_t threads = work <= 128u ? 64u : work <= 256u ? 128u : 256u;
+    // four blocks per SM, as far as a slab has slices: at most with the small blocks, which
+    // pay more for starting than for their slices, at least with those of 256 threads
+    // (at most: B 32 u16 of 381x347x291 50 -> 60 us)
     const uint64_t want = static_cast<uint64_t>(sm_count()) * 4u;
     uint32_t parts = 1;
-    while (parts < p.B && slabs * parts < want) parts *= 2u;
+    while (parts < p.B && (threads < 256u ? slabs * parts * 2u <= want : slabs * parts < want)) parts *= 2u;
     sp.zlen = (p.B + parts - 1) / parts;
     sp.zparts = (p.B + sp.zlen - 1) / sp.zlen;
     sp.items = slabs * sp.zparts;
@@ -923,12 +936,16 @@ static bool launch_brick_slabs(const uint8_t *level, uint8_t *out, const BrickPa
         // call, and another thread's smaller slab must not lower it before this launch
         if (bytes > (48u << 10))
             GC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSlabShared));
-        kernel<<<grid, 256, bytes, s>>>(level, out, sp);
+        kernel<<<grid, threads, bytes, s>>>(level, out, sp);
     };
     if (ch == 16)
-        go(brick_slab_kernel<16>);
+        threads == 64    ? go(brick_slab_kernel<16, 64>)
+        : threads == 128 ? go(brick_slab_kernel<16, 128>)
+                         : go(brick_slab_kernel<16, 256>);
     else
-        go(brick_slab_kernel<8>);
+        threads == 64    ? go(brick_slab_kernel<8, 64>)
+        : threads == 128 ? go(brick_slab_kernel<8, 128>)
+                         : go(brick_slab_kernel<8, 256>);
     GC_CUDA(cudaGetLastError());
     count_launch();
     return true;
