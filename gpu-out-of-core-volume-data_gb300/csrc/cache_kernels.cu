@@ -595,8 +595,10 @@ __global__ void __launch_bounds__(256) brick_bins_kernel(const uint8_t *__restri
 // threads per brick read it 16 bytes a lane with four loads in flight.  Bound by
 // the read of the store.  A warp per brick (G = 32) up to 16 KiB, so that no
 // block barrier follows a brick's few loads; a block above, where one warp would
-// take 64 KiB bricks in 32 dependent turns.  The bricks of a 768^3 u16 volume
-// (16^3, 1.36 GB): 1970 -> 185 us, 7.4 TB/s.
+// take 64 KiB bricks in 32 dependent turns, and for few bricks of more than 2 KiB
+// (warps / blocks: 16^3 floats in big bricks of 2^3, 64 bricks 10.5 / 4.8 us, 512 10.5 /
+// 6.7; 16^3 u8 in big bricks 64 6.2 / 4.4, without 512 4.7 / 6.2).  The bricks of a 768^3 u16
+// volume (16^3, 1.36 GB): 1970 -> 185 us, 7.4 TB/s.
 template <int EB, int G>
 __global__ void __launch_bounds__(256) brick_bins_vec_kernel(const uint8_t *__restrict__ level, uint32_t n,
                                                              uint32_t nbx, uint32_t nby, uint32_t gbx, uint32_t gby,
@@ -654,7 +656,8 @@ void launch_brick_bins(const uint8_t *level, const uint32_t nb[3], const uint32_
     const uint32_t n32 = static_cast<uint32_t>(n);
     if ((B * eb) % 16 == 0 && B <= 512 && reinterpret_cast<uintptr_t>(level) % 16 == 0) {
         const uint32_t cpr = B * eb / 16;
-        const bool warp = B * B * cpr <= 1024;  // 16 KiB
+        const uint32_t chunks = B * B * cpr, sms = static_cast<uint32_t>(sm_count());
+        const bool warp = chunks <= 128 || (chunks <= 1024 && n32 >= sms * (chunks <= 512 ? 2u : 8u));
         auto go = [&](auto kernel) {
             kernel<<<warp ? div_up(n32, 8u) : n32, 256, 0, s>>>(level, n32, nb[0], nb[1], nbig[0], nbig[1], bb[0], bb[1],
                                                                bb[2], B, cpr, bins);
