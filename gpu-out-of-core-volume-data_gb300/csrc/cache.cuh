@@ -137,6 +137,8 @@ struct ViewParams {
     uint32_t eb;                        // bytes per voxel of the view's volume
     uint32_t fallback;                  // sample a coarser mapped level where a brick is missing (preview)
     uint32_t skip_two;                  // step through invisible bricks (DVR, two 8-bit channels)
+    uint32_t *two_rows;                 // ... for each bin of channel 0 the visible bins of channel 1
+                                        // (launch_two_rows)
     uint32_t skip_max;                  // maximum intensity, one channel: step through bricks that cannot
                                         // raise the maximum
     float cell_margin, run_margin;      // margins of the ray caster's run through one brick (run_bound)
@@ -331,8 +333,10 @@ void *march_kernel(uint32_t kind, uint32_t brick_size, bool two_level, MarchShap
 void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s);
 void launch_render(const CacheView &cv, const LevelTables &lt, const ViewParams *views_dev, uint32_t nviews,
                    uint32_t total_tiles, uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);
-// One view, its parameters in the launch; the visible bins are worked out by the
-// ray caster's blocks, for transfer functions of at most kOneViewTf entries.
+// Fills the 32 words of a view's two_rows.
+void launch_two_rows(const ViewParams &view, cudaStream_t s);
+// One view, its parameters in the launch; the visible bins of one channel are worked
+// out by the ray caster's blocks, for transfer functions of at most kOneViewTf entries.
 constexpr uint32_t kOneViewTf = 512;
 void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewParams &view, uint32_t total_tiles,
                        uint32_t rect_tiles, uint32_t *queue, cudaStream_t s);

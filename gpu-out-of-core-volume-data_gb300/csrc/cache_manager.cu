@@ -155,6 +155,9 @@ struct gc_cache {
     uint64_t *status_lru = nullptr, *status_miss = nullptr;
     gc::ScanCtl *ctl_lru = nullptr, *ctl_miss = nullptr;
     uint32_t *d_count = nullptr, *d_misc = nullptr, *d_queue = nullptr;
+    // visible bins of two channels: of the last kTwoRows one-view launches, 32 words each
+    static constexpr uint32_t kTwoRows = 64;
+    uint32_t *d_two_rows = nullptr, two_launches = 0;
     uint4 *d_asked = nullptr, *d_big_coord = nullptr;
     uint32_t *d_owner = nullptr;   // install: lowest list index per page-directory entry (~0 between installs)
     uint64_t *d_coords = nullptr;  // install: page-directory entry per list element
@@ -757,7 +760,7 @@ static void destroy(gc_cache *C) {
     cudaDeviceSynchronize();
     void *dev[] = {C->pt.top, C->pt.table, C->pt.usage, C->pt_order[0], C->pt_order[1], C->pt_keys, C->pt_claim,
                    C->pt_word_of, C->pt_jobs, C->pt_njobs, C->status_pt, C->ctl_pt, C->mrpd, C->req, C->usage, C->order[0], C->order[1], C->slot_level, C->slot_vpos, C->pool, C->slot_bins, C->entry_bins, C->user_bins, C->d_samples,
-                   C->status_lru, C->status_miss, C->ctl_lru, C->ctl_miss, C->d_count, C->d_misc, C->d_queue,
+                   C->status_lru, C->status_miss, C->ctl_lru, C->ctl_miss, C->d_count, C->d_misc, C->d_queue, C->d_two_rows,
                    C->lists[0].d, C->lists[1].d, C->d_asked, C->d_owner, C->d_coords, C->d_big_coord, C->d_big_index, C->d_src,
                    C->d_staging, C->d_views, C->d_cut};
     for (void *p : dev)
@@ -985,6 +988,10 @@ static void render(gc_cache *C, const gc_view *views, uint32_t n, cudaStream_t s
         return;
     }
     if (n == 1 && vp[0].tfw <= kOneViewTf) {
+        if (vp[0].skip_two) {
+            vp[0].two_rows = C->d_two_rows + 32u * (C->two_launches++ % gc_cache::kTwoRows);
+            launch_two_rows(vp[0], s);
+        }
         launch_render_one(cache_view(C), C->lt, vp[0], tiles, rect_total, C->d_queue, s);
         return;
     }
@@ -1174,6 +1181,7 @@ int gc_cache_create_shared(const gc_cache_desc *desc, const gc_volume_desc *volu
         C->d_count = dalloc<uint32_t>(1, "counter");
         C->d_misc = dalloc<uint32_t>(1, "counter");
         C->d_queue = dalloc<uint32_t>(4, "work queue");
+        if (C->nc == 2) C->d_two_rows = dalloc<uint32_t>(32u * gc_cache::kTwoRows, "visible bins of two channels");
         for (auto &L : C->lists) L.d = dalloc<uint4>(maxr, "miss list");
         C->d_asked = dalloc<uint4>(maxr, "asked list");
         C->d_coords = dalloc<uint64_t>(maxr, "install entries");

@@ -1143,11 +1143,11 @@ __global__ void __launch_bounds__(256, N == 2 ? kWideWarps / 8 : 1)
     __shared__ unsigned long long s_visible, s_samples[8], s_rays[8];  // of each warp
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     if (lane == 0) s_samples[warp] = s_rays[warp] = 0;
-    extern __shared__ float4 s_pairs[];  // ONE: 2 (tfw + 4), or 8 tfh with two channels (scratch)
+    extern __shared__ float4 s_pairs[];  // ONE, one channel: 2 (tfw + 4)
     constexpr bool TWO = std::is_same<T, TwoU8>::value;
     __shared__ uint32_t s_two[TWO ? 32 : 1];
     if constexpr (ONE && TWO) {
-        visible_bins_of_two(one, s_two, reinterpret_cast<float *>(s_pairs));
+        if (threadIdx.x < 32u) s_two[threadIdx.x] = one.skip_two ? one.two_rows[threadIdx.x] : ~0u;
         __syncthreads();
     } else if constexpr (ONE) {
         fill_pairs(one.tf, one.tfw, s_pairs);
@@ -1310,6 +1310,19 @@ void launch_view_bins(ViewParams *views_dev, uint32_t n, cudaStream_t s) {
     count_launch();
 }
 
+// Two channels: a launch of its own before the ray caster's.  Worked out by every
+// block of the ray caster instead, the rows took most of a launch whose rays end at
+// once (the passes of a paging loop, frames that have converged): 777x555, tables
+// of 64 x 48 / 256 x 64 / 512 x 64 entries, all rays ended, 36 / 97 / 142 -> 29 / 30 / 30 us.
+__global__ void __launch_bounds__(256) two_rows_kernel(const __grid_constant__ ViewParams view) {
+    visible_row_of_two(view, blockIdx.x, view.two_rows);
+}
+void launch_two_rows(const ViewParams &view, cudaStream_t s) {
+    two_rows_kernel<<<32, 256, 0, s>>>(view);
+    GC_CUDA(cudaGetLastError());
+    count_launch();
+}
+
 // Voxel kind of a cache: its voxel width (1, 2, 4), 0 when its volumes'
 // widths differ, kTwoChannelU8 for two 8-bit channels.
 constexpr uint32_t kTwoChannelU8 = 0x202;
@@ -1381,7 +1394,7 @@ void launch_render_one(const CacheView &cv, const LevelTables &lt, const ViewPar
     const ViewParams *views = nullptr;
     void *args[] = {const_cast<CacheView *>(&cv), const_cast<LevelTables *>(&lt), const_cast<ViewParams *>(&view),
                     &views, &nviews, &total_tiles, &queue, &nwarps};
-    const size_t pairs = cv.nc == 1 ? (view.tfw + 4u) * 2u * sizeof(float4) : (view.skip_two ? view.tfh * 32u * sizeof(float) : 0u);
+    const size_t pairs = cv.nc == 1 ? (view.tfw + 4u) * 2u * sizeof(float4) : 0u;
     GC_CUDA(cudaLaunchKernel(L.func, dim3(L.grid), dim3(L.threads), args, pairs, s));
     count_launch();
 }

@@ -1,4 +1,4 @@
-// Visible value bins of a view (empty-space skipping), by one warp.
+// Visible value bins of a view (empty-space skipping).
 #pragma once
 
 #include "cache.cuh"
@@ -37,45 +37,41 @@ __device__ __forceinline__ unsigned long long visible_bins(const ViewParams &vp,
     return mine;
 }
 
-// Two 8-bit channels and a 2D transfer function, by a block: rows[b] gets the
-// bins of channel 1 that are visible with bin b of channel 0 (32 bins each, the
-// install's).  A sample with its channels in bins b and c reads table entries
-// within the same margins on either axis; the bound is the one above.  scratch:
-// 32 x tfh floats, for each bin of channel 0 the largest alpha of its columns in
-// every row of the table.  A 777x555 frame of 256^3 x 2 voxels 1.90 -> 1.62 ms.
+// Two 8-bit channels and a 2D transfer function of at most kTwoBinRows rows: rows[b]
+// gets the bins of channel 1 that are visible with bin b of channel 0 (32 bins
+// each, the install's), by a block of 256 threads for each b.  A sample with its
+// channels in bins b and c reads table entries within the same margins on either
+// axis; the bound is the one above.  (The skip: a 777x555 frame of 256^3 x 2 voxels
+// 1.90 -> 1.62 ms.)
 constexpr uint32_t kTwoBinRows = 64;  // table rows at most (more: nothing is skipped)
-__device__ __forceinline__ void visible_bins_of_two(const ViewParams &vp, uint32_t *rows, float *scratch) {
-    const uint32_t tid = threadIdx.x, threads = blockDim.x;
-    if (!vp.skip_two) {
-        if (tid < 32u) rows[tid] = ~0u;
-        return;
-    }
+__device__ __forceinline__ void visible_row_of_two(const ViewParams &vp, uint32_t b, uint32_t *rows) {
+    __shared__ float s_row[kTwoBinRows];  // the largest alpha of b's columns in every row of the table
+    const uint32_t lane = threadIdx.x & 31u;
     const int w = static_cast<int>(vp.tfw), h = static_cast<int>(vp.tfh);
-    auto first = [](uint32_t b, int n) {
-        return max(static_cast<int>(floorf(__fadd_rn(__fmul_rn(static_cast<float>(b) / 32.0f, static_cast<float>(n)), -0.5f))) - 1, 0);
+    auto first = [](uint32_t bin, int n) {
+        return max(static_cast<int>(floorf(__fadd_rn(__fmul_rn(static_cast<float>(bin) / 32.0f, static_cast<float>(n)), -0.5f))) - 1, 0);
     };
-    auto last = [](uint32_t b, int n) {
-        return min(static_cast<int>(floorf(__fadd_rn(__fmul_rn(static_cast<float>(b + 1u) / 32.0f, static_cast<float>(n)), -0.5f))) + 2, n - 1);
+    auto last = [](uint32_t bin, int n) {
+        return min(static_cast<int>(floorf(__fadd_rn(__fmul_rn(static_cast<float>(bin + 1u) / 32.0f, static_cast<float>(n)), -0.5f))) + 2, n - 1);
     };
-    if (tid < 32u) rows[tid] = 0u;
-    for (uint32_t k = tid; k < 32u * vp.tfh; k += threads) {
-        const uint32_t b = k & 31u, j = k >> 5;
-        float a = 0.f;
-        const int i1 = last(b, w);
+    const int i0 = first(b, w), i1 = last(b, w);
 #pragma unroll 4
-        for (int i = first(b, w); i <= i1; ++i) a = fmaxf(a, __ldg(vp.tf + 4 * (static_cast<int>(j) * w + i) + 3));
-        scratch[k] = a;
-    }
-    float kmax = 0.f;
-    for (uint32_t l = 0; l < vp.nlevels; ++l) kmax = fmaxf(kmax, vp.kexp[l]);
-    __syncthreads();
-    for (uint32_t k = tid; k < 1024u; k += threads) {
-        const uint32_t b = k & 31u, c = k >> 5;
+    for (int j = static_cast<int>(threadIdx.x >> 5); j < h; j += 8) {
         float a = 0.f;
-        const int j1 = last(c, h);
-        for (int j = first(c, h); j <= j1; ++j) a = fmaxf(a, scratch[32 * j + static_cast<int>(b)]);
-        if (!(a <= 0.04f && __fmul_rn(__fmul_rn(1.05f, kmax), a) < 0.0009f)) atomicOr(rows + b, 1u << c);
+        for (int i = i0 + static_cast<int>(lane); i <= i1; i += 32) a = fmaxf(a, __ldg(vp.tf + 4 * (j * w + i) + 3));
+        // (not negative, so the order of the bits is the order of the values)
+        const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(a));
+        if (lane == 0) s_row[j] = __uint_as_float(m);
     }
+    __syncthreads();
+    if (threadIdx.x >= 32u) return;
+    float kmax = 0.f, a = 0.f;
+    for (uint32_t l = 0; l < vp.nlevels; ++l) kmax = fmaxf(kmax, vp.kexp[l]);
+    const int j1 = last(lane, h);
+    for (int j = first(lane, h); j <= j1; ++j) a = fmaxf(a, s_row[j]);
+    const bool visible = !(a <= 0.04f && __fmul_rn(__fmul_rn(1.05f, kmax), a) < 0.0009f);
+    const uint32_t seen = __ballot_sync(0xffffffffu, visible);
+    if (lane == 0) rows[b] = seen;
 }
 
 }  // namespace gc
