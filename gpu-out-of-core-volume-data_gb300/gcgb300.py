@@ -739,16 +739,16 @@ class Batch:
         self.close()
 
 
-AUTOTUNE_CANDIDATES = [(sched, tw, th, bps) for sched in (1, 0) for tw in (8, 4, 16) for th in (128, 64, 256)
-                       for bps in (0, 4)]
+# scheduler, tile width, threads, blocks per SM (both schedulers launch the same kernel)
+AUTOTUNE_CANDIDATES = [(1, tw, th, bps) for tw in (8, 4, 16) for th in (128, 64, 256) for bps in (0, 4)]
 
 
 def autotune_render(cache, views, clear, stream=0, candidates=None, repeats=3, cache_file=None, key=None,
                     per_view=False):
-    """Chooses the ray caster's launch configuration (scheduler, ray-tile
-    shape, threads per block, blocks per SM) by timing `views` (a list of View
-    whose bricks are resident) under each candidate, applies the fastest and
-    returns (best, timings).  The views render in one launch (the batched
+    """Chooses the ray caster's launch configuration (ray-tile shape, threads
+    per block, blocks per SM; the scheduler has no effect) by timing `views` (a
+    list of View whose bricks are resident) under each candidate, applies the
+    fastest and returns (best, timings).  The views render in one launch (the batched
     form), or with per_view one launch each, timed in sum (the plain per-view
     path).  `clear()` restarts the views' progressive buffers before each timed
     render.  With cache_file and key, a previous choice for the same key is
