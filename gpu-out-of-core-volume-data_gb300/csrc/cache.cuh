@@ -205,7 +205,6 @@ struct ScanCtl {
 };
 
 constexpr uint32_t kErrLookback = 1u;   // a wait for a predecessor's count ran out
-constexpr uint32_t kErrRender = 2u;     // render work-queue wait ran out
 
 // The scans of one frame (frame_scan_kernel): the request scan (nscan > 0) and
 // the used slots of one or two pools.
@@ -294,7 +293,7 @@ void launch_pt_init(uint32_t *order, uint4 *keys, uint32_t nslots, cudaStream_t 
 void launch_brick_bins(const uint8_t *level, const uint32_t nb[3], const uint32_t nbig[3], const uint32_t bb[3],
                        uint32_t B, uint32_t eb, unsigned long long *bins, cudaStream_t s);
 void launch_gather_bricks(const ulonglong2 *src, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,
-                          bool beside, cudaStream_t s);
+                          cudaStream_t s);
 // In-flight marks (page-directory flag 3) of the batched form's overlapped
 // loads: mark the first min(ctl->total, maxreq) entries of a miss list; unmark
 // (3 -> 0) the first n entries of a list after its install.

@@ -1094,8 +1094,9 @@ struct MissedBricks {
                                l.store ? l.bytes : 0u);
     }
 };
-template <typename W, uint32_t kIlp, class Src>
+template <typename W, class Src>
 __device__ __forceinline__ void gather_bricks(const Src src, uint32_t n, uint64_t stride, uint8_t *__restrict__ dst) {
+    constexpr uint32_t kIlp = 2;
     for (uint32_t b = blockIdx.x; b < n; b += gridDim.x) {
         const ulonglong2 e = src(b);
         const W *sp = reinterpret_cast<const W *>(e.x);
@@ -1117,21 +1118,16 @@ __device__ __forceinline__ void gather_bricks(const Src src, uint32_t n, uint64_
         }
     }
 }
-template <typename W>
-__global__ void gather_bricks_kernel(const ulonglong2 *__restrict__ src, uint32_t n, uint64_t stride,
-                                     uint8_t *__restrict__ dst) {
-    gather_bricks<W, 4>(ListedBricks{src}, n, stride, dst);
-}
 // At most 32 registers per thread (128 threads, 16 blocks): fits beside the ray caster.
 template <typename W>
-__global__ void __launch_bounds__(128, 16) gather_bricks_beside_kernel(const ulonglong2 *__restrict__ src, uint32_t n,
-                                                                      uint64_t stride, uint8_t *__restrict__ dst) {
-    gather_bricks<W, 2>(ListedBricks{src}, n, stride, dst);
+__global__ void __launch_bounds__(128, 16) gather_bricks_kernel(const ulonglong2 *__restrict__ src, uint32_t n,
+                                                               uint64_t stride, uint8_t *__restrict__ dst) {
+    gather_bricks<W>(ListedBricks{src}, n, stride, dst);
 }
 template <typename W>
 __global__ void __launch_bounds__(128, 16) gather_missed_kernel(const uint4 *__restrict__ list, const StoreMap m,
                                                                uint32_t n, uint64_t stride, uint8_t *__restrict__ dst) {
-    gather_bricks<W, 2>(MissedBricks{list, m}, n, stride, dst);
+    gather_bricks<W>(MissedBricks{list, m}, n, stride, dst);
 }
 
 void launch_gather_missed(const uint4 *list, const StoreMap &m, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,
@@ -1147,31 +1143,20 @@ void launch_gather_missed(const uint4 *list, const StoreMap &m, uint32_t n, uint
 }
 
 void launch_gather_bricks(const ulonglong2 *src, uint32_t n, uint64_t stride, uint8_t *dst, bool vec16,
-                          bool beside, cudaStream_t s) {
+                          cudaStream_t s) {
     if (n == 0) return;
-    const uint32_t sms = static_cast<uint32_t>(sm_count());
-    if (beside) {
-        // Next to a persistent ray-caster launch: at its occupancy each SM
-        // sub-partition keeps 1024 registers free, room for one warp of 32
-        // registers per thread -- 128-thread blocks (one warp per
-        // sub-partition), one per SM, run during the render instead of after
-        // it (two 16-byte loads in flight per thread).  A second block per
-        // SM, resident before the render's blocks arrive, would hold
-        // registers a ray-caster block needs.
-        const uint32_t grid = std::min<uint32_t>(n, sms);
-        if (vec16)
-            gather_bricks_beside_kernel<uint4><<<grid, 128, 0, s>>>(src, n, stride, dst);
-        else
-            gather_bricks_beside_kernel<uint8_t><<<grid, 128, 0, s>>>(src, n, stride, dst);
-    } else {
-        // alone on the device: one block of 256 per SM (four 16-byte loads in
-        // flight per thread) saturates the host link
-        const uint32_t grid = std::min<uint32_t>(n, sms);
-        if (vec16)
-            gather_bricks_kernel<uint4><<<grid, 256, 0, s>>>(src, n, stride, dst);
-        else
-            gather_bricks_kernel<uint8_t><<<grid, 256, 0, s>>>(src, n, stride, dst);
-    }
+    // Next to a persistent ray-caster launch: at its occupancy each SM
+    // sub-partition keeps 1024 registers free, room for one warp of 32
+    // registers per thread -- 128-thread blocks (one warp per
+    // sub-partition), one per SM, run during the render instead of after
+    // it (two 16-byte loads in flight per thread).  A second block per
+    // SM, resident before the render's blocks arrive, would hold
+    // registers a ray-caster block needs.
+    const uint32_t grid = std::min<uint32_t>(n, static_cast<uint32_t>(sm_count()));
+    if (vec16)
+        gather_bricks_kernel<uint4><<<grid, 128, 0, s>>>(src, n, stride, dst);
+    else
+        gather_bricks_kernel<uint8_t><<<grid, 128, 0, s>>>(src, n, stride, dst);
     GC_CUDA(cudaGetLastError());
     count_launch();
 }

@@ -496,7 +496,7 @@ static void resolve_and_upload(gc_cache *C, uint32_t n) {
     GC_CUDA(cudaEventRecord(C->ev_upload_begin, s));
     if (nhost && gather) {
         GC_CUDA(cudaMemcpyAsync(C->d_src, C->h_src, nbig * sizeof(ulonglong2), cudaMemcpyHostToDevice, s));
-        launch_gather_bricks(C->d_src, nbig, C->big_stride, C->d_staging, C->vec16, true, s);
+        launch_gather_bricks(C->d_src, nbig, C->big_stride, C->d_staging, C->vec16, s);
     } else if (nhost) {
         GC_CUDA(cudaMemcpyAsync(C->d_staging, C->h_staging, static_cast<size_t>(nbig) * C->big_stride,
                                 cudaMemcpyHostToDevice, s));
@@ -1403,7 +1403,7 @@ int gc_brick_value_bins(const gc_volume_desc *vol, const gc_layout *layout, uint
         const uint32_t *nb = layout->nb_bricks[level];
         const uint64_t n = static_cast<uint64_t>(nb[0]) * nb[1] * nb[2];
         cudaStream_t s = as_stream(stream);
-        if (vol->channels != 1) {  // the install never skips a multi-channel brick
+        if (vol->channels != 1) {  // the user's bins are of one channel: such a brick is always requested
             GC_CUDA(cudaMemsetAsync(bins, 0xff, n * sizeof(uint64_t), s));
             return;
         }
