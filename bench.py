@@ -102,9 +102,9 @@ PIXEL_BYTES = 44  # RGBA 4 + t 4+4 + colour state 16+16 per pixel and launch
 # DRAM bytes (read + write) of the c2 roofline launch (view 42, converged, after
 # an L2 flush), from one ncu capture of this command:
 #   ncu --set full --clock-control none --nvtx --nvtx-include roofline/ -k regex:render_kernel -c 1
-#       python bench.py --roofline-only --steps 3 --tuning 0,16,128,0
+#       python bench.py --roofline-only --steps 3 --tuning 1,16,128,0
 # (profiles/render_kernel_c2_1024x1024.md).  None for the other configs.
-ROOFLINE_TRAFFIC = {"c2": 106_319_872}
+ROOFLINE_TRAFFIC = {"c2": 107_634_944}
 BRICK_BINS = {}  # value bins of every brick, by brick-store address
 
 
