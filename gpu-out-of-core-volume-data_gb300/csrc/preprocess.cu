@@ -259,13 +259,14 @@ static void launch_mip(const void *src, void *dst, const uint32_t d[3], uint32_t
     // windows of 16 bytes from a number of threads on, below which a thread per value
     // fills the SMs better.  Windows / a thread per value, at threads of eight bytes
     // out: u8 17k 6.1 / 4.2 us, 28k 6.0 / 4.3, 38k 6.1 / 6.2, 80k 6.3 / 8.2; u16 31k 5.4 /
-    // 4.1, 41k 6.0 / 4.3, 54k 6.1 / 6.0, 158k 6.3 / 8.2; two 16-bit channels 45k 5.6 / 4.3,
-    // 61k 5.6 / 6.2; two 8-bit channels, whose values are smaller and twice as many,
-    // 17k 4.7 / 4.1, 23k 5.7 / 4.3, 32k 5.2 / 6.0, 72k 6.2 / 7.0; four 32k 4.6 / 6.1.  Floats (a voxel
-    // is a load either way) a thread per value at every size: 500k 41 / 39 us.
+    // 4.1, 41k 6.0 / 4.3, 49k 6.1 / 5.2, 54k 6.1 / 6.0, 158k 6.3 / 8.2; two 16-bit channels
+    // 45k 5.6 / 4.3, 61k 5.6 / 6.2; two 8-bit channels, whose values are smaller and twice
+    // as many, 17k 4.7 / 4.1, 23k 5.7 / 4.3, 32k 5.2 / 6.0, 72k 6.2 / 7.0; four 32k 4.6 /
+    // 6.1.  Floats (a voxel is a load either way) a thread per value at every size: 500k
+    // 41 / 39 us.
     p.chunks = static_cast<uint32_t>((p.out_row + 7) / 8);
     p.total = static_cast<uint64_t>(p.chunks) * p.oY * p.oZ;
-    if (p.total >= (cb == 1 && nc > 1 ? 28672u : 49152u) && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
+    if (p.total >= (cb == 1 && nc > 1 ? 28672u : 53248u) && reinterpret_cast<uintptr_t>(src) % 16 == 0 &&
         reinterpret_cast<uintptr_t>(dst) % eb == 0 &&
         ((cb == 1 && (nc == 1 || nc == 2 || nc == 4)) || (cb == 2 && nc <= 2))) {
         const auto go = [&](auto kernel) {

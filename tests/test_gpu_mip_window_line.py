@@ -25,15 +25,15 @@ def check(gc, t, rng, dims, eb, ch, real=False):
 @pytest.mark.parametrize("eb,ch", [(1, 1), (2, 1), (4, 2)])
 def test_short_rows_above_the_line(gc, torch_cuda, eb, ch):
     rng = np.random.default_rng(eb + ch)
-    for X in list(range(2, 36)) + [61, 127]:  # 350 x 151 rows out: above the line from one chunk a row on
-        check(gc, torch_cuda, rng, (X, 700, 303), eb, ch)
+    for X in list(range(2, 36)) + [61, 127]:  # 360 x 151 rows out: above the line from one chunk a row on
+        check(gc, torch_cuda, rng, (X, 720, 303), eb, ch)
 
 
 @pytest.mark.parametrize("eb,ch,real", [(1, 1, False), (2, 1, False), (4, 2, False), (2, 2, False), (4, 4, False),
                                         (4, 1, True)])
 def test_sizes_beside_the_line(gc, torch_cuda, eb, ch, real):
     rng = np.random.default_rng(7 * eb + ch)
-    line = 28672 if eb == ch and ch > 1 else 49152
+    line = 28672 if eb == ch and ch > 1 else 53248
     for X in (3, 9, 17, 33, 67):
         chunks = (X // 2 * eb + 7) // 8
         for rows in (line // (chunks * 64) - 1, line // (chunks * 64), line // (chunks * 64) + 1):
