@@ -1079,17 +1079,18 @@ __global__ void __launch_bounds__(256) empty_warp_kernel(const uint4 *__restrict
 // (up to 8, as far as the bricks fill the SMs), a warp first looks at the first 512
 // bytes of each, and the whole block reads those that this leaves open.  4,854 big
 // bricks of 108 KiB dense / half of them empty / all empty, value by value 6.6 / 433 /
-// 760, a block each without the look (16 KiB of every brick) 15 / 46 / 79, with it 5.5 /
-// 46 / 82 us; 1,024 of 32 KiB 4.5 / 27 / 27, 5.7 / 6.5 / 6.8, 4.4 / 6.8 / 8.5 us.
-template <int CB>
+// 760, a block each without the look (16 KiB of every brick) 15 / 46 / 79, with it 5.6 /
+// 46 / 82 us; 1,024 of 32 KiB 4.5 / 27 / 27, 5.6 / 6.5 / 6.8, 4.4 / 6.8 / 8.5 us.  Up to
+// four per SM no look (kLook): 16 KiB of each cost nothing there, the look 1 us.
+template <int CB, bool kLook>
 __global__ void __launch_bounds__(256) empty_block_kernel(const uint4 *__restrict__ bricks, uint64_t nbig,
                                                           uint64_t chunks, uint32_t per, float threshold,
                                                           uint8_t *__restrict__ flags) {
     __shared__ uint32_t s_open[8];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint64_t b0 = static_cast<uint64_t>(blockIdx.x) * per;
-    bool open = false;
-    if (warp < per && b0 + warp < nbig) {
+    bool open = !kLook && warp < per && b0 + warp < nbig;
+    if (kLook && warp < per && b0 + warp < nbig) {
         open = !__any_sync(0xffffffffu, reaches<CB, 32>(bricks + (b0 + warp) * chunks, 0, lane, 32, threshold));
         if (!open && lane == 0) flags[b0 + warp] = 0;
     }
@@ -1208,13 +1209,19 @@ int gc_bricks_empty(const void *bricks, uint64_t nb_big_bricks, const gc_volume_
                 };
                 cb == 1 ? go(empty_warp_kernel<1>) : cb == 2 ? go(empty_warp_kernel<2>) : go(empty_warp_kernel<4>);
             } else {
+                const bool look = nb_big_bricks > sms * 4;
                 const uint32_t per =
                     static_cast<uint32_t>(std::max<uint64_t>(1, std::min<uint64_t>(8, nb_big_bricks / (sms * 8))));
                 const unsigned blocks = static_cast<unsigned>((nb_big_bricks + per - 1) / per);
                 auto go = [&](auto kernel) {
                     kernel<<<blocks, 256, 0, as_stream(stream)>>>(in, nb_big_bricks, bytes / 16, per, threshold, flags);
                 };
-                cb == 1 ? go(empty_block_kernel<1>) : cb == 2 ? go(empty_block_kernel<2>) : go(empty_block_kernel<4>);
+                if (cb == 1)
+                    look ? go(empty_block_kernel<1, true>) : go(empty_block_kernel<1, false>);
+                else if (cb == 2)
+                    look ? go(empty_block_kernel<2, true>) : go(empty_block_kernel<2, false>);
+                else
+                    look ? go(empty_block_kernel<4, true>) : go(empty_block_kernel<4, false>);
             }
             GC_CUDA(cudaGetLastError());
             count_launch();

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 # bytes of a big brick: 32 KiB (B 32), 128 KiB, 256 KiB; numbers around one block per
 # big brick, several, and a warp each
-@pytest.mark.parametrize("cb,B,n", [(1, 32, 1), (1, 32, 1217), (1, 32, 2433), (1, 32, 7295), (1, 32, 7297), (2, 32, 2433),
+@pytest.mark.parametrize("cb,B,n", [(1, 32, 1), (1, 32, 608), (1, 32, 609), (1, 32, 1217), (1, 32, 2433), (1, 32, 7295), (1, 32, 7297), (2, 32, 2433),
                                     (4, 32, 41), (4, 32, 2433), (1, 64, 2433), (2, 40, 2431)])
 def test_one_value_anywhere(gc, torch_cuda, cb, B, n):
     t = torch_cuda
