@@ -231,9 +231,10 @@ void launch_frame_scan(FrameScan a, const LevelTables &lt, cudaStream_t s);
 void launch_lru_partition(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
                           uint32_t nslots, const uint32_t *count, uint64_t *status, ScanCtl *ctl, cudaStream_t s);
 // The LRU update of a pool of at most kClusterSlots slots, used slots counted too.
-// An update with its request scan, cluster / count + partition: 4,096 slots 15.2 /
-// 16.2 us, 32,768 15.0 / 16.9, 65,536 14.4 / 16.8, 131,072 16.9 / 17.1; 262,144
-// (32 slots a thread) 19.3 / 18.0.
+// An update with its request scan, cluster / count beside the scan + partition: 32,768
+// slots 15.2 / 14.8 us, 65,536 15.2 / 15.5, 131,072 17.7 / 17.2; an update without it
+// (install frames) saves the count's launch up to here.  262,144 slots (32 a thread)
+// 19.3 / 18.0.
 constexpr uint32_t kClusterSlots = 131072;
 void launch_lru_cluster(const uint32_t *order_in, uint32_t *order_out, const uint32_t *usage, uint32_t ts,
                         uint32_t nslots, uint32_t *count, cudaStream_t s);
